@@ -1,0 +1,36 @@
+// Launcher of the marching-warps RK4 iteration (phx_step_march.cuh), compiled
+// in its own unit (phx_march.cu).
+#pragma once
+
+#include <array>
+#include <map>
+
+#include "phx_rt.hpp"
+
+namespace phx {
+
+struct MarchOptions {
+    bool res = true;     // reservoir
+    bool fma = false;    // fused multiply-add arithmetic (FP32)
+    bool store = false;  // also write the stage values (FusedParams::st_psi / st_n)
+    bool pdl = true;     // programmatic stream serialization
+};
+
+template <typename T>
+class MarchLauncher {
+public:
+    // planes of `plane` points can be indexed in 32 bits
+    static bool fits(long long plane) { return plane < (1LL << 31); }
+    // one iteration F.psi0, F.n0 -> F.psi1, F.n1 on `stream` of the current device
+    void launch(const FusedParams<T>& F, const MarchOptions& o, int sm_count, cudaStream_t stream);
+
+private:
+    std::map<const void*, int> per_sm_;  // CTAs per SM of the kernel variants used so far
+    std::array<int, 4> plan_{};          // grid, CTAs per SM and SMs of the last row segmentation
+    int plan_rows_ = 0;
+};
+
+extern template class MarchLauncher<float>;
+extern template class MarchLauncher<double>;
+
+}  // namespace phx

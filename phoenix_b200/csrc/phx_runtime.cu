@@ -39,6 +39,7 @@
 #include "phx_step_stream.cuh"
 #include "phx_step_tetm_fused.cuh"
 #include "phx_rt.hpp"
+#include "phx_march.hpp"
 #include "phx_adjoint.cuh"
 #include "phx_ssfm.cuh"
 #include "phx_dp45_fused.cuh"
@@ -136,7 +137,7 @@ struct Engine final : EngineBase {
     static constexpr int kTuneIters = 3;   // consecutive iterations of one candidate per sample
     static constexpr double kTuneMargin = 0.03;  // a challenger must beat the incumbent by this fraction
     static constexpr int kFusedShape = kShapes;  // launch shapes 4-7: whole RK4 iteration in one kernel
-    static constexpr int kFusedShapes = 11;      // shapes 8-13: persistent TMA-fed tiles, 14: column strips
+    static constexpr int kFusedShapes = 11;      // shapes 8-13: persistent TMA-fed tiles (12: marching warps), 14: column strips
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> tune_ev[kShapes + kFusedShapes];
     static constexpr int kRingBlocks = 256;  // blocks of the ring-norm kernels (their partial-sum slots follow the stage kernels')
     static constexpr int kNormBlocks = 296;
@@ -845,6 +846,16 @@ struct Engine final : EngineBase {
         const int blocks = (int)std::min<long long>(Q.n_segs, slots);
         launch_pdl(kern, dim3(blocks), dim3(NT), Lay::total, Q);
     }
+    // ---- marching warps (phx_step_march.cuh)
+    MarchLauncher<T> march;
+    void go_march(const FusedParams<T>& F, bool res, bool fma) {
+        if (!sm_count) PHX_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, P.device));
+        MarchOptions o;
+        o.res = res;
+        o.fma = fma;
+        o.pdl = pdl_on();
+        march.launch(F, o, sm_count, stream);
+    }
     void check_err_flag() {
         if (!err_flag.p) return;
         int v = 0;
@@ -866,7 +877,13 @@ struct Engine final : EngineBase {
             case 6: go_tma<RES, 64, f32 ? 16 : 8, 384, 2, FMA>(F); return;
             // taller tiles, one CTA per SM: less halo recomputation per output point
             case 7: go_tma<RES, 64, f32 ? 32 : 16, 768, 1, FMA>(F); return;
-            case 8: go_tma<RES, 64, f32 ? 32 : 16, 512, 1, FMA>(F); return;
+            // marching warps; planes that 32 bits cannot index take the incumbent
+            case 8:
+                if (MarchLauncher<T>::fits(plane))
+                    go_march(F, RES, FMA);
+                else
+                    go_tma<RES, 64, f32 ? 16 : 8, 384, 2, FMA>(F);
+                return;
             // 64 x 14: 1024^2 makes 1184 tiles, exactly four rounds of 296 CTAs
             // (64 x 16 leaves the fourth round half empty)
             case 9: go_tma<RES, 64, f32 ? 14 : 7, 384, 2, FMA>(F); return;

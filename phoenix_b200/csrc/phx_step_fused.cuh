@@ -60,8 +60,9 @@ constexpr int kImg = kImgDepth;
 // ((g_r n) * (-i psi), (R/2 n) * psi, (V c) * (-i psi)); this keeps only the
 // products that are not with that zero, which changes no result except,
 // possibly, the sign of an exact zero.
-// (PP: any parameter struct with these constants and per-stage pump_c / pot_c)
-template <typename T, bool RES, typename PP>
+// (PP: any parameter struct with these constants and per-stage pump_c / pot_c.
+// UNIT: the caller knows every pump_c / pot_c to be exactly 1.)
+template <typename T, bool RES, bool UNIT = false, typename PP>
 __device__ __forceinline__ void rhs_fused(const PP& P, int s, cx<T> in_wf, cx<T> up, cx<T> dn, cx<T> left,
                                           cx<T> right, T in_rv, T pump, T pot, bool has_pump, bool has_pot, cx<T>& k_wf,
                                           T& k_rv) {
@@ -75,10 +76,10 @@ __device__ __forceinline__ void rhs_fused(const PP& P, int s, cx<T> in_wf, cx<T>
         wf = cadd(wf, smul(rmul(P.ohb_gr, in_rv), in_wf_mi));
         wf = cadd(wf, smul(rmul(P.half_R, in_rv), in_wf));
         T krv = rmul(-radd(P.gamma_r, rmul(P.R, in_psi_norm)), in_rv);
-        if (has_pump) krv = radd(krv, rmul(pump, P.pump_c[s]));
+        if (has_pump) krv = radd(krv, UNIT ? pump : rmul(pump, P.pump_c[s]));
         k_rv = krv;
     }
-    if (has_pot) wf = cadd(wf, smul(rmul(P.ohb, rmul(pot, P.pot_c[s])), in_wf_mi));
+    if (has_pot) wf = cadd(wf, smul(rmul(P.ohb, UNIT ? pot : rmul(pot, P.pot_c[s])), in_wf_mi));
     k_wf = wf;
 }
 
@@ -95,7 +96,7 @@ __device__ __forceinline__ void rhs_fused(const PP& P, int s, cx<T> in_wf, cx<T>
 __device__ __forceinline__ float fm(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fm(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-template <typename T, bool RES>
+template <typename T, bool RES, bool UNIT = false>
 __device__ __forceinline__ void rhs_fma(const FusedParams<T>& P, int s, cx<T> psi, cx<T> up, cx<T> dn, cx<T> left,
                                         cx<T> right, T n, T pump, T pot, bool has_pump, bool has_pot, cx<T>& k, T& kn) {
     const T norm = fm(psi.re, psi.re, rmul(psi.im, psi.im));
@@ -108,25 +109,25 @@ __device__ __forceinline__ void rhs_fma(const FusedParams<T>& P, int s, cx<T> ps
         W = fm(P.ohb_gr, n, W);
         B = fm(P.half_R, n, B);
     }
-    if (has_pot) W = fm(rmul(P.ohb, P.pot_c[s]), pot, W);
+    if (has_pot) W = fm(UNIT ? P.ohb : rmul(P.ohb, P.pot_c[s]), pot, W);
     const T A = rmul(P.ohb, P.meff);
     k.re = fm(A, lim, fm(W, psi.im, rmul(B, psi.re)));
     k.im = fm(-A, lre, fm(-W, psi.re, rmul(B, psi.im)));
     if constexpr (RES) {
         const T g = fm(P.R, norm, P.gamma_r);
-        kn = has_pump ? fm(-g, n, rmul(pump, P.pump_c[s])) : rmul(-g, n);
+        kn = has_pump ? fm(-g, n, UNIT ? pump : rmul(pump, P.pump_c[s])) : rmul(-g, n);
     }
 }
 
 // the right-hand side of stage s in the chosen arithmetic
-template <typename T, bool RES, bool FMA>
+template <typename T, bool RES, bool FMA, bool UNIT = false>
 __device__ __forceinline__ void rhs_iter(const FusedParams<T>& P, int s, cx<T> in_wf, cx<T> up, cx<T> dn, cx<T> left,
                                          cx<T> right, T in_rv, T pump, T pot, bool has_pump, bool has_pot, cx<T>& k_wf,
                                          T& k_rv) {
     if constexpr (FMA)
-        rhs_fma<T, RES>(P, s, in_wf, up, dn, left, right, in_rv, pump, pot, has_pump, has_pot, k_wf, k_rv);
+        rhs_fma<T, RES, UNIT>(P, s, in_wf, up, dn, left, right, in_rv, pump, pot, has_pump, has_pot, k_wf, k_rv);
     else
-        rhs_fused<T, RES>(P, s, in_wf, up, dn, left, right, in_rv, pump, pot, has_pump, has_pot, k_wf, k_rv);
+        rhs_fused<T, RES, UNIT>(P, s, in_wf, up, dn, left, right, in_rv, pump, pot, has_pump, has_pot, k_wf, k_rv);
 }
 // y + a k
 template <bool FMA, typename T>

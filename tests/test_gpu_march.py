@@ -1,0 +1,69 @@
+"""The marching-warps RK4 iteration (launch shape 12): strips store 56 columns
+(two points per lane), row segments end anywhere.  Against the stage kernels
+(shape 2), bit for bit, and in the fused multiply-add arithmetic against the
+tile kernels (shape 4)."""
+import itertools
+
+import numpy as np
+import pytest
+
+import bench as B
+import phoenix_b200 as pb
+
+pytestmark = pytest.mark.gpu
+
+# columns around one and two strips (56, 112), the smallest grid, odd FP64
+# widths; rows of one short segment and of several
+SIZES = [(8, 8), (10, 9), (54, 37), (56, 12), (58, 140), (112, 35), (114, 301), (250, 97)]
+ODD = [(9, 8), (55, 41), (57, 33), (113, 150)]
+
+
+def run(n_c, n_r, dtype, px, py, shape, monkeypatch, res=True, pump=True, pot=True, temporal=False, fma=False, iters=5):
+    monkeypatch.setenv("PHX_STAGE_SHAPE", str(shape))
+    rng = np.random.default_rng([n_c, n_r])
+    T = pb.Temporal
+    sp = pb.SystemParameters(N_c=n_c, N_r=n_r, L_x=0.3 * n_c, L_y=0.2 * n_r, **B.PHYS, periodic_boundary_x=px,
+                             periodic_boundary_y=py, dtype=dtype, dt=0.01, t_max=1e12, fft_every=1e12, use_reservoir=res,
+                             pump_temporal=[T("cos", 0.02, 0.05, 40.0) if temporal else T()] if pump and res else [],
+                             potential_temporal=[T("gauss", 0.02, 0.05, 1.0) if temporal else T()] if pot else [], fma=fma)
+    psi0 = rng.standard_normal((n_r, n_c)) + 1j * rng.standard_normal((n_r, n_c))
+    with pb.Solver(sp) as s:
+        s.set_field("psi_plus", psi0)
+        if res:
+            s.set_field("n_plus", rng.random((n_r, n_c)))
+            if pump:
+                s.set_field("pump_plus", 2.0 * rng.random((n_r, n_c)), 0)
+        if pot:
+            s.set_field("potential_plus", 0.3 * rng.standard_normal((n_r, n_c)), 0)
+        info = s.run(iters)
+        assert info.launch_shape == shape
+        return [s.get_field("psi_plus")] + ([s.get_field("n_plus")] if res else [])
+
+
+@pytest.mark.parametrize("px,py", list(itertools.product([True, False], repeat=2)))
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+def test_edges_of_strips_and_segments(require_gpu, monkeypatch, dtype, px, py):
+    for n_c, n_r in SIZES + (ODD if dtype == "f64" else []):
+        want = run(n_c, n_r, dtype, px, py, 2, monkeypatch)
+        for a, b in zip(run(n_c, n_r, dtype, px, py, 12, monkeypatch), want):
+            np.testing.assert_array_equal(a, b, err_msg=f"{n_c} x {n_r}")
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+@pytest.mark.parametrize("res,pump,pot,temporal", [(False, False, False, False), (False, False, True, False),
+                                                   (True, False, False, False), (True, True, False, False),
+                                                   (True, False, True, False), (True, True, False, True),
+                                                   (True, True, True, True), (False, False, True, True)])
+def test_inputs_and_envelopes(require_gpu, monkeypatch, dtype, res, pump, pot, temporal):
+    a = run(114, 70, dtype, True, False, 12, monkeypatch, res, pump, pot, temporal)
+    b = run(114, 70, dtype, True, False, 2, monkeypatch, res, pump, pot, temporal)
+    for x, y in zip(a, b):
+        np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("res,pot,temporal", [(True, True, False), (True, False, False), (True, True, True), (False, True, False)])
+def test_fma_arithmetic(require_gpu, monkeypatch, res, pot, temporal):
+    a = run(114, 70, "f32", True, True, 12, monkeypatch, res, True, pot, temporal, fma=True)
+    b = run(114, 70, "f32", True, True, 4, monkeypatch, res, True, pot, temporal, fma=True)
+    for x, y in zip(a, b):
+        np.testing.assert_array_equal(x, y)
