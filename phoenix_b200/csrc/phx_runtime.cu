@@ -252,6 +252,10 @@ struct Engine final : EngineBase {
         result.alloc(sizeof(double) * 4, stream);
         host_result.alloc(sizeof(double) * 4);
         imag_f.alloc(sizeof(double) * 2, stream);
+        // set up here, not at the first launch that needs it: check_err_flag
+        // reads it past the stream's queue, and must never see what the
+        // memory held before
+        if (fused_eligible_static()) err_flag.alloc(sizeof(int), stream);
         t = (T)P.t0;
         dt = (T)P.dt;
         fft_cached_t = (T)0.0;
@@ -738,7 +742,6 @@ struct Engine final : EngineBase {
     template <int TW, int TH>
     void prepare_tma(TmaParams<T>& Q, const FusedParams<T>& F) {
         static_assert(TW % 4 == 0, "TMA box x alignment needs tile origins on 16-byte boundaries");
-        if (!err_flag.p) err_flag.alloc(sizeof(int), stream);
         std::memset(&Q, 0, sizeof(Q));
         Q.f = F;
         // tensor maps over whole allocations (padded (0,0) = interior (-G,-G));
@@ -803,7 +806,6 @@ struct Engine final : EngineBase {
             PHX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, kern, NT, Lay::total));
             if (blocks_per_sm < 1) fail(PHX_ERR_UNSUPPORTED, "column-strip iteration kernel does not fit on an SM");
         }
-        if (!err_flag.p) err_flag.alloc(sizeof(int), stream);
         if (!sm_count) PHX_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, P.device));
         auto map_of = [&](const void* base, bool complex) -> const CUtensorMap& {
             const auto key = std::make_tuple(base, complex, TW + 8, TH);
@@ -2072,7 +2074,6 @@ struct Engine final : EngineBase {
             PHX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, kern, NT, Lay::total));
             if (blocks_per_sm < 1) fail(PHX_ERR_UNSUPPORTED, "TMA iteration kernel does not fit on an SM");
         }
-        if (!err_flag.p) err_flag.alloc(sizeof(int), stream);
         if (!sm_count) PHX_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, P.device));
         // a map depends on the plane's address, on whether it is complex and
         // on the box (the tile shape); pitch and rows are fixed for the handle

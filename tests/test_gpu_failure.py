@@ -124,3 +124,24 @@ def test_abort_request_stops_a_running_step(require_gpu):
         # the request was consumed: the handle keeps stepping
         assert s.run(3).iterations == 3
         assert np.isfinite(s.sum_abs2("psi_plus"))
+
+
+def test_a_new_handle_does_not_read_what_its_error_flag_held_before(require_gpu, monkeypatch):
+    """A handle that is still tuning (non-TMA shapes first, TMA shapes later) is
+    read back while its iterations are queued: the flag of the bounded waits
+    starts at zero, whatever an earlier handle left in that memory."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("PHX_TUNE_CACHE", "0")
+    monkeypatch.delenv("PHX_STAGE_SHAPE", raising=False)
+    psi, pump = _inputs(512)
+    psi_t = torch.from_numpy(psi).cuda()
+    for _ in range(4):
+        # leaves nonzero sums in its small device buffers
+        with pb.Solver(_system(512, iterator="DP45", use_adaptive_timestep=True, tolerance=1e-6, dtype="f64", dt_min=1e-6)) as s:
+            _load(s, psi, pump)
+            s.run(3)
+        with pb.Solver(_system(512, dtype="f64")) as s:
+            _load(s, psi, pump)
+            s.set_field_tensor("psi_plus", psi_t)
+            s.run(50)
+            assert torch.isfinite(torch.view_as_real(s.get_field_tensor("psi_plus"))).all()
