@@ -6,8 +6,9 @@
 // (layout of phx_device.cuh), parameters and clock, and one batch iteration
 // advances every instance by one RK4 iteration (the fused iteration of
 // phx_step_fused.cuh, bit-identical to a single-simulation handle) in a
-// single launch of the persistent TMA kernel rk4_batch_kernel, which walks
-// the tiles of all instances through a tile -> instance table.  Launch
+// single launch: of the persistent TMA kernel rk4_batch_kernel, which walks
+// the tiles of all instances through a tile -> instance table, or of marching
+// warps (phx_step_march.cuh) over all instances' row segments.  Launch
 // sequences are captured once into CUDA graphs and replayed.
 #include <cuda_runtime.h>
 
@@ -26,29 +27,32 @@
 #include "phx_rt.hpp"
 #include "phx_step_fused.cuh"
 #include "phx_step_tma.cuh"
+#include "phx_march.hpp"
 
 namespace phx {
 
-// Tile shapes the batch autotuner chooses from: TW x TH points, NT threads.
+// Launch shapes the batch autotuner chooses from: tiles of TW x TH points, NT
+// threads, and (kBatchMarch) marching warps (phx_step_march.cuh), no tiles.
 // FP64 tiles are half as high (shared memory of the two TMA slots).
 // MINB: CTAs per SM the register allocation leaves room for (the 12-warp
 // shapes run two per SM).
 constexpr int kBatchShapes = 5;
+constexpr int kBatchMarch = 2;
 template <typename T>
 struct BatchShape;
 template <>
 struct BatchShape<float> {
-    static constexpr int TW[kBatchShapes] = {32, 64, 32, 32, 64};
-    static constexpr int TH[kBatchShapes] = {32, 16, 16, 32, 16};
-    static constexpr int NT[kBatchShapes] = {256, 256, 128, 384, 384};
-    static constexpr int MINB[kBatchShapes] = {1, 1, 1, 2, 2};
+    static constexpr int TW[kBatchShapes] = {32, 64, 0, 32, 64};
+    static constexpr int TH[kBatchShapes] = {32, 16, 0, 32, 16};
+    static constexpr int NT[kBatchShapes] = {256, 256, 0, 384, 384};
+    static constexpr int MINB[kBatchShapes] = {1, 1, 0, 2, 2};
 };
 template <>
 struct BatchShape<double> {
-    static constexpr int TW[kBatchShapes] = {32, 64, 32, 32, 64};
-    static constexpr int TH[kBatchShapes] = {16, 8, 8, 16, 8};
-    static constexpr int NT[kBatchShapes] = {256, 256, 128, 384, 384};
-    static constexpr int MINB[kBatchShapes] = {1, 1, 1, 2, 2};
+    static constexpr int TW[kBatchShapes] = {32, 64, 0, 32, 64};
+    static constexpr int TH[kBatchShapes] = {16, 8, 0, 16, 8};
+    static constexpr int NT[kBatchShapes] = {256, 256, 0, 384, 384};
+    static constexpr int MINB[kBatchShapes] = {1, 1, 0, 2, 2};
 };
 
 struct BatchBase {
@@ -87,6 +91,7 @@ struct BatchEngine final : BatchBase {
     DevBuf d_inst[kBatchShapes], d_tile[kBatchShapes];
     int n_tiles[kBatchShapes] = {};
     int blocks[kBatchShapes] = {};
+    MarchBatch<T> march;
     DevBuf err_flag;
     int sm_count = 0;
 
@@ -235,10 +240,18 @@ struct BatchEngine final : BatchBase {
         if (per_sm < 1) fail(PHX_ERR_UNSUPPORTED, "batch iteration kernel does not fit on an SM");
         blocks[S] = std::max(1, std::min(n_tiles[S], per_sm * sm_count));
     }
+    void build_march() {
+        std::vector<BatchInstance<T>> hi;
+        std::vector<int> tiles;
+        table<0>(hi, tiles);
+        std::vector<FusedParams<T>> f;
+        for (const auto& b : hi) f.insert(f.end(), {b.f[0], b.f[1]});
+        march.build(f, res, fma, sm_count, stream);
+    }
     void build_tables() {
         build_one<0>();
         build_one<1>();
-        build_one<2>();
+        build_march();
         build_one<3>();
         build_one<4>();
         static_assert(kBatchShapes == 5, "every shape needs its tables");
@@ -260,7 +273,7 @@ struct BatchEngine final : BatchBase {
         switch (sh) {
             case 0: go<0>(dir); break;
             case 1: go<1>(dir); break;
-            case 2: go<2>(dir); break;
+            case kBatchMarch: march.launch(dir, stream); break;
             case 3: go<3>(dir); break;
             default: go<4>(dir); break;
         }

@@ -13,30 +13,44 @@ namespace {
 // schedulers waiting on one warp's latencies).  More CTAs than fit at once
 // follow one another without a common end, hence the fractional rounds.
 template <typename T>
-int march_seg_rows(int N_r, int strips, int per_sm, int sm_count) {
+double march_cost(int L, long long items, int per_sm, int sm_count) {
     const double cost32[4] = {0.0, 0.61, 0.86, 1.2}, cost64[3] = {0.0, 0.94, 1.55};
     auto cost = [&](int w) {
         if (sizeof(T) == 4) return w <= 3 ? cost32[w] : cost32[3] * w / 3;
         return w <= 2 ? cost64[w] : cost64[2] * w / 2;
     };
-    int best_L = N_r;
+    const long long ctas = (items + kMarchWarps - 1) / kMarchWarps, w = (ctas + sm_count - 1) / sm_count;
+    return (L + 3.0) *
+           (w <= per_sm ? cost((int)w) : ((double)ctas / ((double)per_sm * sm_count) + 0.3) * cost(per_sm));
+}
+// the cheapest segment length of at most max_rows, items(L) segments in all
+template <typename T, typename Items>
+int march_seg_rows(int max_rows, const Items& items, int per_sm, int sm_count) {
+    int best_L = max_rows;
     double best = -1.0;
-    for (int L = std::min(N_r, 2); L <= std::min(N_r, 256); ++L) {
-        const long long items = (long long)strips * ((N_r + L - 1) / L);
-        const long long ctas = (items + kMarchWarps - 1) / kMarchWarps;
-        const long long w = (ctas + sm_count - 1) / sm_count;
-        const double t = (L + 3.0) * (w <= per_sm ? cost((int)w)
-                                                  : ((double)ctas / ((double)per_sm * sm_count) + 0.3) * cost(per_sm));
+    for (int L = std::min(max_rows, 2); L <= std::min(max_rows, 256); ++L) {
+        const double t = march_cost<T>(L, items(L), per_sm, sm_count);
         if (best < 0.0 || t < best) best = t, best_L = L;
     }
     return best_L;
 }
+template <typename K>
+int march_occupancy(K kern, int bytes) {
+    int per_sm = 0;
+    PHX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    PHX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kMarchWarps, bytes));
+    if (per_sm < 1) fail(PHX_ERR_UNSUPPORTED, "marching iteration kernel does not fit on an SM");
+    return per_sm;
+}
+// CTAs per SM the registers must leave room for (FP32 150, FP64 250 registers)
+template <typename T>
+constexpr int kMarchMinB = sizeof(T) == 4 ? 3 : 2;
 
 }  // namespace
 
 template <typename T>
 void MarchLauncher<T>::launch(const FusedParams<T>& F, const MarchOptions& o, int sm_count, cudaStream_t stream) {
-    constexpr int MINB = sizeof(T) == 4 ? 3 : 2;  // FP32 150, FP64 250 registers
+    constexpr int MINB = kMarchMinB<T>;
     using Lay = MarchLayout<T>;
     using K = void (*)(MarchParams<T>);
     bool unit = true;
@@ -71,17 +85,14 @@ void MarchLauncher<T>::launch(const FusedParams<T>& F, const MarchOptions& o, in
     }
     if (!kern) fail(PHX_ERR_UNSUPPORTED, "the fused multiply-add arithmetic is FP32 only");
     int& per_sm = per_sm_[reinterpret_cast<const void*>(kern)];
-    if (!per_sm) {
-        PHX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::bytes));
-        PHX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kMarchWarps, Lay::bytes));
-        if (per_sm < 1) fail(PHX_ERR_UNSUPPORTED, "marching iteration kernel does not fit on an SM");
-    }
+    if (!per_sm) per_sm = march_occupancy(kern, Lay::bytes);
     MarchParams<T> Q;
     Q.f = F;
     Q.strips = (F.N_c + kMarchOut - 1) / kMarchOut;
     const std::array<int, 4> plan = {F.N_r, F.N_c, per_sm, sm_count};
     if (plan != plan_) {
-        plan_rows_ = march_seg_rows<T>(F.N_r, Q.strips, per_sm, sm_count);
+        plan_rows_ = march_seg_rows<T>(
+            F.N_r, [&](int L) { return (long long)Q.strips * ((F.N_r + L - 1) / L); }, per_sm, sm_count);
         plan_ = plan;
     }
     Q.seg_rows = plan_rows_;
@@ -99,6 +110,68 @@ void MarchLauncher<T>::launch(const FusedParams<T>& F, const MarchOptions& o, in
     PHX_CUDA(cudaLaunchKernelEx(&cfg, kern, Q));
 }
 
+template <typename T>
+void MarchBatch<T>::build(const std::vector<FusedParams<T>>& f, bool res, bool fma, int sm_count, cudaStream_t stream) {
+    using K = void (*)(MarchBatchParams<T>);
+    constexpr int MINB = kMarchMinB<T>;
+    bool pot = false;
+    int max_rows = 1;
+    const int n = (int)(f.size() / 2);
+    for (int i = 0; i < n; ++i) {
+        pot = pot || f[2 * i].pot != nullptr;
+        max_rows = std::max(max_rows, f[2 * i].N_r);
+    }
+    K kern = nullptr;
+    auto pick = [&](auto m) {
+        constexpr bool M = decltype(m)::value;
+        if (res)
+            kern = pot ? (K)rk4_march_batch_kernel<T, true, true, M, MINB> : (K)rk4_march_batch_kernel<T, true, false, M, MINB>;
+        else
+            kern = pot ? (K)rk4_march_batch_kernel<T, false, true, M, MINB> : (K)rk4_march_batch_kernel<T, false, false, M, MINB>;
+    };
+    if constexpr (sizeof(T) == 4) {
+        if (fma) pick(std::true_type{});
+    }
+    if (!kern) pick(std::false_type{});
+    const int per_sm = march_occupancy(kern, MarchLayout<T>::bytes);
+    auto strips = [&](int i) { return (f[2 * i].N_c + kMarchOut - 1) / kMarchOut; };
+    const int L = march_seg_rows<T>(
+        max_rows,
+        [&](int l) {
+            long long items = 0;
+            for (int i = 0; i < n; ++i) items += (long long)strips(i) * ((f[2 * i].N_r + l - 1) / l);
+            return items;
+        },
+        per_sm, sm_count);
+    std::vector<MarchItem> items;
+    for (int i = 0; i < n; ++i) {
+        const int rows = f[2 * i].N_r, segs = (rows + L - 1) / L, per = (rows + segs - 1) / segs;
+        for (int r = 0; r < rows; r += per)
+            for (int s = 0; s < strips(i); ++s) items.push_back({i, s, r, std::min(r + per, rows)});
+    }
+    f_.alloc(sizeof(FusedParams<T>) * f.size(), stream);
+    items_.alloc(sizeof(MarchItem) * items.size(), stream);
+    PHX_CUDA(cudaMemcpyAsync(f_.p, f.data(), f_.bytes, cudaMemcpyHostToDevice, stream));
+    PHX_CUDA(cudaMemcpyAsync(items_.p, items.data(), items_.bytes, cudaMemcpyHostToDevice, stream));
+    PHX_CUDA(cudaStreamSynchronize(stream));  // the host vectors die here
+    kern_ = reinterpret_cast<const void*>(kern);
+    n_items_ = (int)items.size();
+}
+
+template <typename T>
+void MarchBatch<T>::launch(int dir, cudaStream_t stream) const {
+    MarchBatchParams<T> Q;
+    Q.f = static_cast<const FusedParams<T>*>(f_.p);
+    Q.items = static_cast<const MarchItem*>(items_.p);
+    Q.n_items = n_items_;
+    Q.dir = dir;
+    void* args[] = {&Q};
+    PHX_CUDA(cudaLaunchKernel(kern_, dim3((unsigned)((n_items_ + kMarchWarps - 1) / kMarchWarps)), dim3(32 * kMarchWarps), args,
+                              MarchLayout<T>::bytes, stream));
+}
+
+template class MarchBatch<float>;
+template class MarchBatch<double>;
 template class MarchLauncher<float>;
 template class MarchLauncher<double>;
 

@@ -4,6 +4,7 @@
 
 #include <array>
 #include <map>
+#include <vector>
 
 #include "phx_rt.hpp"
 
@@ -30,6 +31,22 @@ private:
     int plan_rows_ = 0;
 };
 
+// The same iteration over every instance of a batch, in one launch.
+template <typename T>
+class MarchBatch {
+public:
+    // f: two directions per instance (constant envelopes); waits for the copies
+    void build(const std::vector<FusedParams<T>>& f, bool res, bool fma, int sm_count, cudaStream_t stream);
+    void launch(int dir, cudaStream_t stream) const;
+
+private:
+    DevBuf f_, items_;
+    const void* kern_ = nullptr;
+    int n_items_ = 0;
+};
+
+extern template class MarchBatch<float>;
+extern template class MarchBatch<double>;
 extern template class MarchLauncher<float>;
 extern template class MarchLauncher<double>;
 

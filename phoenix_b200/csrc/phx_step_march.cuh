@@ -102,28 +102,26 @@ __device__ __forceinline__ void ring_two(const unsigned char* p, double* v) {
     v[0] = u.x, v[1] = u.y;
 }
 
+// One warp's segment: rows [R0, R1) of strip `strip`; `ring` is the warp's
+// shared memory.
 // POT: the potential's terms are evaluated (an absent plane counts as zero).
 // UNIT: every temporal coefficient is exactly 1 (constant envelopes); the
 // products with it, which change nothing, are left out.  STORE: also write
 // the stage values Y2..Y4 of the stored points (with periodic images), which
 // the adjoint's backward sweep reads.  Plane indices are 32-bit (the host
 // takes this kernel for planes of fewer than 2^31 points only).
-template <typename T, bool RES, bool POT, bool UNIT, bool FMA, bool STORE, int MINB>
-__global__ void __launch_bounds__(32 * kMarchWarps, MINB) rk4_march_kernel(const __grid_constant__ MarchParams<T> Q) {
+template <typename T, bool RES, bool POT, bool UNIT, bool FMA, bool STORE>
+__device__ __forceinline__ void march_segment(const FusedParams<T>& P, int strip, int R0, int R1, unsigned char* ring) {
     using Lay = MarchLayout<T>;
     using C = cx<T>;
     constexpr int CPT = 2;
-    extern __shared__ __align__(16) unsigned char march_smem[];
-    const FusedParams<T>& P = Q.f;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int item = blockIdx.x * kMarchWarps + warp;
-    if (item >= Q.n_items) return;
-    const int strip = item % Q.strips, seg = item / Q.strips;
-    const int R0 = seg * Q.seg_rows, R1 = min(R0 + Q.seg_rows, P.N_r);
+    // the RK4 weights (FusedParams::b)
+    constexpr T wb[4] = {(T)(1.0 / 6.0), (T)(1.0 / 3.0), (T)(1.0 / 3.0), (T)(1.0 / 6.0)};
+    const int lane = threadIdx.x & 31;
     const int c = strip * kMarchOut - 4 + CPT * lane;
     const int pitch = (int)P.pitch;
     const bool has_pump = RES && P.pump != nullptr, has_pot = POT && P.pot != nullptr;
-    unsigned char* const mine = march_smem + warp * Lay::warp_bytes + lane * 16;
+    unsigned char* const mine = ring + lane * 16;
     if ((RES && !has_pump) || (POT && !has_pot)) {
         for (int k = 0; k < kMarchRing; ++k)
 #pragma unroll
@@ -157,10 +155,6 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB) rk4_march_kernel(const
         next_g += next_k < last_k ? pitch : 0;
         ++next_k;
     };
-    // The next iteration's kernel is scheduled when this one's CTAs are done, not
-    // earlier: CTAs that wait in free slots leave the next grid unevenly spread
-    // over the SMs (25.4 against 18.6 us at 1024^2 FP32, two CTAs per SM).
-    pdl_wait();
 #pragma unroll
     for (int k = 0; k < 5; ++k) issue();
 
@@ -244,18 +238,18 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB) rk4_march_kernel(const
             T tn = (T)0;
             on[j] = (T)0;
             if constexpr (s == 0) {
-                t = smul(P.b[0], kw[j]);
-                tn = rmul(P.b[0], kn[j]);
+                t = smul(wb[0], kw[j]);
+                tn = rmul(wb[0], kn[j]);
             } else if constexpr (s < 3) {
-                t = axpy<FMA>(P.b[s], kw[j], a[before][j]);
-                tn = raxpy<FMA>(P.b[s], kn[j], an[before][j]);
+                t = axpy<FMA>(wb[s], kw[j], a[before][j]);
+                tn = raxpy<FMA>(wb[s], kn[j], an[before][j]);
             }
             if constexpr (s < 3) {
                 o[j] = axpy<FMA>(P.dtw[own], kw[j], y0[j]);
                 if constexpr (RES) on[j] = raxpy<FMA>(P.dtw[own], kn[j], n0[j]);
             } else {
-                o[j] = final_update<FMA>(P.dt, P.b[3], a[2][j], kw[j], y0[j]);
-                if constexpr (RES) on[j] = rfinal_update<FMA>(P.dt, P.b[3], an[2][j], kn[j], n0[j]);
+                o[j] = final_update<FMA>(P.dt, wb[3], a[2][j], kw[j], y0[j]);
+                if constexpr (RES) on[j] = rfinal_update<FMA>(P.dt, wb[3], an[2][j], kn[j], n0[j]);
             }
             // what stage s - 1 handed on for this row is used up: the next row's takes its place
             if constexpr (s > 0) a[before][j] = pa[j], an[before][j] = pan[j], ns[before][j] = pn[j];
@@ -309,6 +303,45 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB) rk4_march_kernel(const
     // the last rows' copies may still be on their way: they must land before
     // the CTA's shared memory can belong to another kernel's
     cp_async_wait<0>();
+}
+
+template <typename T, bool RES, bool POT, bool UNIT, bool FMA, bool STORE, int MINB>
+__global__ void __launch_bounds__(32 * kMarchWarps, MINB) rk4_march_kernel(const __grid_constant__ MarchParams<T> Q) {
+    extern __shared__ __align__(16) unsigned char march_smem[];
+    const int warp = threadIdx.x >> 5, item = blockIdx.x * kMarchWarps + warp;
+    if (item >= Q.n_items) return;
+    const int R0 = item / Q.strips * Q.seg_rows;
+    // The previous iteration's kernel has completed.  The next one's is
+    // scheduled when this one's CTAs are done, not earlier: CTAs that wait in
+    // free slots leave the next grid unevenly spread over the SMs (25.4 against
+    // 18.6 us at 1024^2 FP32, two CTAs per SM).
+    pdl_wait();
+    march_segment<T, RES, POT, UNIT, FMA, STORE>(Q.f, item % Q.strips, R0, min(R0 + Q.seg_rows, Q.f.N_r),
+                                                 march_smem + warp * MarchLayout<T>::warp_bytes);
+}
+
+// ---------------------------------------------------------------- batches
+// The segments of every instance of a batch, one warp each.  An instance's
+// constants are loaded into registers once per segment.
+struct MarchItem {
+    int inst, strip, r0, r1;
+};
+
+template <typename T>
+struct MarchBatchParams {
+    const FusedParams<T>* f;  // [instance][direction]
+    const MarchItem* items;
+    int n_items, dir;
+};
+
+template <typename T, bool RES, bool POT, bool FMA, int MINB>
+__global__ void __launch_bounds__(32 * kMarchWarps, MINB) rk4_march_batch_kernel(const __grid_constant__ MarchBatchParams<T> Q) {
+    extern __shared__ __align__(16) unsigned char march_smem[];
+    const int warp = threadIdx.x >> 5, item = blockIdx.x * kMarchWarps + warp;
+    if (item >= Q.n_items) return;
+    const MarchItem it = Q.items[item];
+    const FusedParams<T> P = Q.f[2 * it.inst + Q.dir];
+    march_segment<T, RES, POT, true, FMA, false>(P, it.strip, it.r0, it.r1, march_smem + warp * MarchLayout<T>::warp_bytes);
 }
 
 }  // namespace phx
