@@ -1,9 +1,10 @@
 // Split-step Fourier iterator (the reference's "SSFM",
 // source/cuda_solver/solver/iterator/split_step_fourier_method.cu:24-72 with
-// the kernels of include/kernel/kernel_gp_compute.cuh:244-440).  Halo 0: the
-// wavefunction is worked on as a contiguous N_r x N_c array between four
+// the kernels of include/kernel/kernel_gp_compute.cuh:244-440).  Halo 0: four
 // unnormalised cuFFT transforms per iteration, with the (N_c, N_r) plan of
-// solver_fft.cu:102-118; the reservoir stays in its halo-padded plane.
+// solver_fft.cu:102-118.  Square grids are transformed in place on the
+// halo-padded planes; other shapes as a contiguous N_r x N_c copy, which that
+// plan reads as N_c rows of N_r.  The reservoir stays in its padded plane.
 //   linear half step   psi <- F^-1[ F[psi] / N2 exp(-i lin dt / 2) ],
 //                      lin = hbar / 2 / m (kx^2 + ky^2), k = 2 pi j / L with
 //                      the reference's literal pi = 3.1415926535
@@ -25,6 +26,7 @@ template <typename T>
 struct SsfmParams {
     int N_r, N_c;
     long long pitch;     // of the padded planes
+    long long wp;        // row pitch of the transformed arrays: N_c, or pitch (in place on the padded planes)
     int tetm, res;
     T hbs, meff, Lx, Ly, dt, N2;
     T g_c, g_r, R, gamma_c, gamma_r, g_pm, ohb, dV;
@@ -51,21 +53,32 @@ __device__ __forceinline__ cx<T> cexp_dev(cx<T> z) {
     return mk(e * c, e * s);
 }
 
-// gp_scalar_linear_fourier: out = in / N2 * exp(minus_i * lin * dt / 2)
+// exp(minus_i * lin * dt / 2) of every k-space point: a table, since lin and dt
+// are the same in every iteration (the exponential with its double divisions
+// took longer than the transforms it sits between)
 template <typename T>
-__global__ void ssfm_linear_kernel(const __grid_constant__ SsfmParams<T> S, const cx<T>* __restrict__ in,
-                                   cx<T>* __restrict__ out) {
+__global__ void ssfm_table_kernel(const __grid_constant__ SsfmParams<T> S, cx<T>* __restrict__ table) {
     const long long N = (long long)S.N_r * S.N_c;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-        const T row = (T)(unsigned)(i / S.N_c), col = (T)(unsigned)(i % S.N_c);
+        const T row = (T)((unsigned)i / (unsigned)S.N_c), col = (T)((unsigned)i % (unsigned)S.N_c);
         const T kx = (T)(2.0 * 3.1415926535 * (double)(col <= (T)((unsigned)S.N_c / 2) ? col : -(T)S.N_c + col) / (double)S.Lx);
         const T ky = (T)(2.0 * 3.1415926535 * (double)(row <= (T)((unsigned)S.N_r / 2) ? row : -(T)S.N_r + row) / (double)S.Ly);
         const T lin = (T)((double)S.hbs / 2.0 / (double)S.meff * (double)radd(rmul(kx, kx), rmul(ky, ky)));
         cx<T> z = mk(rmul((T)0.0, lin), rmul((T)-1.0, lin));
         z = mk(rmul(z.re, S.dt), rmul(z.im, S.dt));
         z = mk(rdiv(z.re, (T)2.0), rdiv(z.im, (T)2.0));
-        const cx<T> a = in[i];
-        out[i] = cmul(mk(rdiv(a.re, S.N2), rdiv(a.im, S.N2)), cexp_dev(z));
+        table[i] = cexp_dev(z);
+    }
+}
+// gp_scalar_linear_fourier: out = in / N2 * table; rows of S.wp points
+template <typename T>
+__global__ void ssfm_linear_kernel(const __grid_constant__ SsfmParams<T> S, const cx<T>* table, const cx<T>* in, cx<T>* out) {
+    const long long N = (long long)S.N_r * S.N_c;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
+        const unsigned r = (unsigned)i / (unsigned)S.N_c, c = (unsigned)i - r * (unsigned)S.N_c;  // at most 2^31 points
+        const long long w = r * S.wp + c;
+        const cx<T> a = in[w];
+        out[w] = cmul(mk(rdiv(a.re, S.N2), rdiv(a.im, S.N2)), table[i]);
     }
 }
 
@@ -103,28 +116,27 @@ __device__ __forceinline__ void ssfm_nonlinear_one(const SsfmParams<T>& S, int c
 
 // gp_scalar_nonlinear: (fft, rv) -> (wf, buffer rv)
 template <typename T>
-__global__ void ssfm_nonlinear_kernel(const __grid_constant__ SsfmParams<T> S, const cx<T>* __restrict__ fp,
-                                      const cx<T>* __restrict__ fm, const T* __restrict__ rvp, const T* __restrict__ rvm,
-                                      cx<T>* __restrict__ wp, cx<T>* __restrict__ wm, T* __restrict__ brvp,
-                                      T* __restrict__ brvm) {
+__global__ void ssfm_nonlinear_kernel(const __grid_constant__ SsfmParams<T> S, const cx<T>* fp, const cx<T>* fm,
+                                      const T* rvp, const T* rvm, cx<T>* wp, cx<T>* wm, T* brvp, T* brvm) {
     const long long N = (long long)S.N_r * S.N_c;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-        const long long r = i / S.N_c, c = i - r * S.N_c, pi = r * S.pitch + c;
+        const unsigned r = (unsigned)i / (unsigned)S.N_c, c = (unsigned)i - r * (unsigned)S.N_c;  // at most 2^31 points
+        const long long pi = r * S.pitch + c, w = r * S.wp + c;
         if (!S.tetm) {
             cx<T> o;
             T on;
-            ssfm_nonlinear_one(S, 0, pi, fp[i], S.res ? rvp[pi] : (T)0, (T)0, o, on);
-            wp[i] = o;
+            ssfm_nonlinear_one(S, 0, pi, fp[w], S.res ? rvp[pi] : (T)0, (T)0, o, on);
+            wp[w] = o;
             if (S.res) brvp[pi] = on;
         } else {
-            const cx<T> a = fp[i], b = fm[i];
+            const cx<T> a = fp[w], b = fm[w];
             cx<T> o;
             T on;
             ssfm_nonlinear_one(S, 0, pi, a, rvp[pi], abs2(b), o, on);
-            wp[i] = o;
+            wp[w] = o;
             brvp[pi] = on;
             ssfm_nonlinear_one(S, 1, pi, b, rvm[pi], abs2(a), o, on);
-            wm[i] = o;
+            wm[w] = o;
             brvm[pi] = on;
         }
     }
@@ -133,12 +145,12 @@ __global__ void ssfm_nonlinear_kernel(const __grid_constant__ SsfmParams<T> S, c
 // gp_scalar_independent: psi = fft + pulse + dw into the padded state plane;
 // the scalar branch copies the buffer reservoir back, the TE/TM branch does not
 template <typename T>
-__global__ void ssfm_independent_kernel(const __grid_constant__ SsfmParams<T> S, const cx<T>* __restrict__ fp,
-                                        const cx<T>* __restrict__ fm, T* __restrict__ rvp, const T* __restrict__ brvp,
-                                        const T* __restrict__ brvm, cx<T>* __restrict__ psip, cx<T>* __restrict__ psim) {
+__global__ void ssfm_independent_kernel(const __grid_constant__ SsfmParams<T> S, const cx<T>* fp,
+                                        const cx<T>* fm, T* rvp, const T* brvp, const T* brvm, cx<T>* psip, cx<T>* psim) {
     const long long N = (long long)S.N_r * S.N_c;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-        const long long r = i / S.N_c, c = i - r * S.N_c, pi = r * S.pitch + c;
+        const unsigned r = (unsigned)i / (unsigned)S.N_c, c = (unsigned)i - r * (unsigned)S.N_c;  // at most 2^31 points
+        const long long pi = r * S.pitch + c, w = r * S.wp + c;
         cx<T> ap = mk((T)0, (T)0), am = mk((T)0, (T)0);
         for (int k = 0; k < S.n_pulse; ++k) {
             if (!S.tetm) {
@@ -159,8 +171,8 @@ __global__ void ssfm_independent_kernel(const __grid_constant__ SsfmParams<T> S,
                 am = cadd(am, mk(rmul(xi.re, scm), rmul(xi.im, scm)));
             }
         }
-        psip[pi] = cadd(fp[i], ap);
-        if (S.tetm) psim[pi] = cadd(fm[i], am);
+        psip[pi] = cadd(fp[w], ap);
+        if (S.tetm) psim[pi] = cadd(fm[w], am);
         else if (S.res) rvp[pi] = brvp[pi];
     }
 }
