@@ -77,7 +77,8 @@ def build_host(force: bool = False, verbose: bool = False) -> None:
             os.symlink(os.path.basename(CLI_BIN), link)
 
 
-UNITS = ["phx_runtime.cu", "phx_noalloc.cu", "phx_batch.cu", "phx_march.cu"]
+UNITS = ["phx_runtime.cu", "phx_noalloc.cu", "phx_batch.cu", "phx_march.cu",
+         "phx_march_general.cu"]
 OBJ_DIR = os.path.join(PKG, "_build")
 
 

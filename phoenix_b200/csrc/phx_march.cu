@@ -2,46 +2,12 @@
 // launch.
 #include "phx_march.hpp"
 
+#include "phx_march_plan.hpp"
 #include "phx_step_march.cuh"
 
 namespace phx {
 namespace {
 
-// Rows per segment.  A segment of L rows costs about L + 3 full steps (its
-// first rows run through some stages only), and an SM with w CTAs takes
-// cost[w] per step of all of them (measured at 1024^2; one CTA leaves its
-// schedulers waiting on one warp's latencies).  More CTAs than fit at once
-// follow one another without a common end, hence the fractional rounds.
-template <typename T>
-double march_cost(int L, long long items, int per_sm, int sm_count) {
-    const double cost32[4] = {0.0, 0.61, 0.86, 1.2}, cost64[3] = {0.0, 0.94, 1.55};
-    auto cost = [&](int w) {
-        if (sizeof(T) == 4) return w <= 3 ? cost32[w] : cost32[3] * w / 3;
-        return w <= 2 ? cost64[w] : cost64[2] * w / 2;
-    };
-    const long long ctas = (items + kMarchWarps - 1) / kMarchWarps, w = (ctas + sm_count - 1) / sm_count;
-    return (L + 3.0) *
-           (w <= per_sm ? cost((int)w) : ((double)ctas / ((double)per_sm * sm_count) + 0.3) * cost(per_sm));
-}
-// the cheapest segment length of at most max_rows, items(L) segments in all
-template <typename T, typename Items>
-int march_seg_rows(int max_rows, const Items& items, int per_sm, int sm_count) {
-    int best_L = max_rows;
-    double best = -1.0;
-    for (int L = std::min(max_rows, 2); L <= std::min(max_rows, 256); ++L) {
-        const double t = march_cost<T>(L, items(L), per_sm, sm_count);
-        if (best < 0.0 || t < best) best = t, best_L = L;
-    }
-    return best_L;
-}
-template <typename K>
-int march_occupancy(K kern, int bytes) {
-    int per_sm = 0;
-    PHX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    PHX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kMarchWarps, bytes));
-    if (per_sm < 1) fail(PHX_ERR_UNSUPPORTED, "marching iteration kernel does not fit on an SM");
-    return per_sm;
-}
 // CTAs per SM the registers must leave room for (FP32 150, FP64 250 registers)
 template <typename T>
 constexpr int kMarchMinB = sizeof(T) == 4 ? 3 : 2;
@@ -97,17 +63,7 @@ void MarchLauncher<T>::launch(const FusedParams<T>& F, const MarchOptions& o, in
     }
     Q.seg_rows = plan_rows_;
     Q.n_items = Q.strips * ((F.N_r + Q.seg_rows - 1) / Q.seg_rows);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((Q.n_items + kMarchWarps - 1) / kMarchWarps));
-    cfg.blockDim = dim3(32 * kMarchWarps);
-    cfg.dynamicSmemBytes = Lay::bytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = o.pdl ? 1 : 0;
-    PHX_CUDA(cudaLaunchKernelEx(&cfg, kern, Q));
+    march_launch(kern, Q, Q.n_items, Lay::bytes, stream, o.pdl);
 }
 
 template <typename T>

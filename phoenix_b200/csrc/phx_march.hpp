@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "phx_rt.hpp"
+#include "phx_stage_tetm.cuh"
 
 namespace phx {
 
@@ -45,6 +46,27 @@ private:
     int n_items_ = 0;
 };
 
+// The iteration with noise, pulses, a second pump group or two polarisations
+// (phx_step_march_general.cuh, compiled in phx_march_general.cu).
+template <typename T>
+class MarchGeneral {
+public:
+    // st: the parameters of the four stages (scalar model: .p only); state
+    // planes per component.  False when no variant takes this iteration.
+    bool launch(const TetmParams<T> (&st)[4], int comps, bool res, const cx<T>* const* psi0, const T* const* n0,
+                cx<T>* const* psi1, T* const* n1, int sm_count, cudaStream_t stream, bool pdl);
+
+private:
+    template <int COMPS>
+    bool launch_comps(const TetmParams<T> (&st)[4], const cx<T>* const* psi0, const T* const* n0, cx<T>* const* psi1,
+                      T* const* n1, int sm_count, cudaStream_t stream, bool pdl);
+    std::map<const void*, int> per_sm_;  // CTAs per SM of the kernel variants used so far
+    std::array<int, 4> plan_{};          // grid, CTAs per SM and SMs of the last row segmentation
+    int plan_rows_ = 0;
+};
+
+extern template class MarchGeneral<float>;
+extern template class MarchGeneral<double>;
 extern template class MarchBatch<float>;
 extern template class MarchBatch<double>;
 extern template class MarchLauncher<float>;

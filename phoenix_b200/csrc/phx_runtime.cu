@@ -165,7 +165,7 @@ struct Engine final : EngineBase {
     DevBuf pump[2], pot[2], pulse[2];  // input planes (groups)
     DevBuf mask[2];                    // fft-shifted mask, contiguous N_r*N_c
     DevBuf fft_x;                      // contiguous scratch for the filter
-    DevBuf psi_alt, n_alt;             // second state plane for the fused RK4 iteration
+    DevBuf psi_alt[2], n_alt[2];       // second state planes of the one-kernel RK4 iterations
     DevBuf err_flag;                   // set by kernels whose bounded waits gave up
     DevBuf partials, result;
     PinnedBuf host_result;
@@ -536,6 +536,7 @@ struct Engine final : EngineBase {
         S.noise_amp = noise_amp;
         S.dV = d.dV;
         S.four_dV = (T)4.0 * d.dV;
+        S.inv_dV = (T)1.0 / d.dV;
         S.gamma_c = (T)P.gamma_c;
         S.noise_scale = std::sqrt((T)P.gamma_c / S.four_dV);
         S.imag = imag_time() ? 1 : 0;
@@ -926,15 +927,12 @@ struct Engine final : EngineBase {
                 F.pot_c[s] = c.real();
             }
         }
-        if (!psi_alt.p) {
-            psi_alt.alloc(sizeof(C) * plane, stream);
-            n_alt.alloc(sizeof(T) * plane, stream);
-        }
+        ensure_alt();
         fused_constants<T>(F, P, d, dt, pitch);
         F.psi0 = cplane(psi[0]);
         F.n0 = rplane(nres[0]);
-        F.psi1 = cplane(psi_alt);
-        F.n1 = rplane(n_alt);
+        F.psi1 = cplane(psi_alt[0]);
+        F.n1 = rplane(n_alt[0]);
         F.pump = P.n_pump_groups ? rplane(pump[0]) : nullptr;
         F.pot = P.n_potential_groups ? rplane(pot[0]) : nullptr;
         cudaEvent_t a = nullptr;
@@ -961,9 +959,39 @@ struct Engine final : EngineBase {
                  pts * (2 * st + (P.n_pump_groups ? sizeof(T) : 0) + (P.n_potential_groups ? sizeof(T) : 0)));
         ++launches;
         PHX_CUDA(cudaGetLastError());
-        std::swap(psi[0].p, psi_alt.p);
-        std::swap(nres[0].p, n_alt.p);
+        swap_alt();
         return true;
+    }
+    // The one-kernel iterations write the other of two state planes, and of its
+    // ring only the periodic images: the zeros along zero axes stay.
+    void ensure_alt() {
+        for (int q = 0; q < comps; ++q)
+            if (!psi_alt[q].p) {
+                psi_alt[q].alloc(sizeof(C) * plane, stream);
+                n_alt[q].alloc(sizeof(T) * plane, stream);
+            }
+    }
+    void swap_alt() {
+        for (int q = 0; q < comps; ++q) {
+            std::swap(psi[q].p, psi_alt[q].p);
+            std::swap(nres[q].p, n_alt[q].p);
+        }
+    }
+    // the marching-warps form of an iteration the kernels below also take
+    MarchGeneral<T> march_general;
+    bool go_march_general(const TetmParams<T> (&st)[4]) {
+        if (!sm_count) PHX_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, P.device));
+        const C* p0[2] = {};
+        const T* n0[2] = {};
+        C* p1[2] = {};
+        T* n1[2] = {};
+        for (int q = 0; q < comps; ++q) {
+            p0[q] = cplane(psi[q]);
+            n0[q] = rplane(nres[q]);
+            p1[q] = cplane(psi_alt[q]);
+            n1[q] = rplane(n_alt[q]);
+        }
+        return march_general.launch(st, comps, P.use_reservoir != 0, p0, n0, p1, n1, sm_count, stream, pdl_on());
     }
 
     // ---- TE/TM: the whole iteration in one kernel (phx_step_tetm_fused.cuh);
@@ -988,6 +1016,7 @@ struct Engine final : EngineBase {
         const T cw[4] = {(T)0.0, (T)0.5, (T)0.5, (T)1.0};
         const T aw[3] = {(T)0.5, (T)0.5, (T)1.0};
         const T bw[4] = {(T)(1.0 / 6.0), (T)(1.0 / 3.0), (T)(1.0 / 3.0), (T)(1.0 / 6.0)};
+        ensure_alt();
         TetmFusedParams<T> F;
         std::memset(&F, 0, sizeof(F));
         for (int s = 1; s <= 4; ++s) {
@@ -1009,22 +1038,24 @@ struct Engine final : EngineBase {
         for (int q = 0; q < 2; ++q) {
             F.psi0[q] = cplane(psi[q]);
             F.n0[q] = rplane(nres[q]);
-            F.psi1[q] = cplane(sbuf_psi[q][0]);
-            F.n1[q] = rplane(sbuf_n[q][0]);
+            F.psi1[q] = cplane(psi_alt[q]);
+            F.n1[q] = rplane(n_alt[q]);
         }
         cudaEvent_t a = nullptr;
         prof_begin(a);
-        if constexpr (sizeof(T) == 4)
-            go_tetm_fused<32, 16, 512>(F);
-        else
-            go_tetm_fused<32, 8, 512>(F);
+        if (!go_march_general(F.st)) {
+            if constexpr (sizeof(T) == 4)
+                go_tetm_fused<32, 16, 512>(F);
+            else
+                go_tetm_fused<32, 8, 512>(F);
+        }
         // read psi, n (both components) + pump, potential per group; write psi, n
         const double pt = 2.0 * (2.0 * sizeof(C) + 2.0 * sizeof(T)) +
                           2.0 * sizeof(T) * (P.n_pump_groups + P.n_potential_groups) + 2.0 * sizeof(C) * P.n_pulse_groups;
         prof_end(PHX_KERNEL_RK4_FUSED, a, pt * (double)N_r * N_c);
         ++launches;
         PHX_CUDA(cudaGetLastError());
-        swap_state_with(0);
+        swap_alt();
     }
 
     // ---- scalar RK4 with what rk4_tma_kernel does not take (noise, pulses,
@@ -1053,8 +1084,9 @@ struct Engine final : EngineBase {
         const T cw[4] = {(T)0.0, (T)0.5, (T)0.5, (T)1.0};
         const T aw[3] = {(T)0.5, (T)0.5, (T)1.0};
         const T bw[4] = {(T)(1.0 / 6.0), (T)(1.0 / 3.0), (T)(1.0 / 3.0), (T)(1.0 / 6.0)};
-        ScalarFusedParams<T> F;
-        std::memset(&F, 0, sizeof(F));
+        ensure_alt();
+        TetmParams<T> st[4];
+        std::memset(st, 0, sizeof(st));
         for (int s = 1; s <= 4; ++s) {
             // the per-stage kernels' parameters of stage s (step_rk4 below)
             StageParams<T> S = base_params(0);
@@ -1066,25 +1098,29 @@ struct Engine final : EngineBase {
             S.pump = rplane(pump[0]);
             S.pot = rplane(pot[0]);
             S.pulse = cplane(pulse[0]);
-            F.st[s - 1] = S;
+            st[s - 1].p = S;
         }
-        F.psi0 = cplane(psi[0]);
-        F.n0 = rplane(nres[0]);
-        F.psi1 = cplane(sbuf_psi[0][0]);
-        F.n1 = rplane(sbuf_n[0][0]);
         cudaEvent_t a = nullptr;
         prof_begin(a);
-        constexpr bool f32 = sizeof(T) == 4;
-        if (P.use_reservoir)
-            go_general<true, 32, f32 ? 16 : 8, 512>(F);
-        else
-            go_general<false, 32, f32 ? 16 : 8, 512>(F);
+        if (!go_march_general(st)) {
+            ScalarFusedParams<T> F;
+            for (int s = 0; s < 4; ++s) F.st[s] = st[s].p;
+            F.psi0 = cplane(psi[0]);
+            F.n0 = rplane(nres[0]);
+            F.psi1 = cplane(psi_alt[0]);
+            F.n1 = rplane(n_alt[0]);
+            constexpr bool f32 = sizeof(T) == 4;
+            if (P.use_reservoir)
+                go_general<true, 32, f32 ? 16 : 8, 512>(F);
+            else
+                go_general<false, 32, f32 ? 16 : 8, 512>(F);
+        }
         const double pt = 2.0 * (sizeof(C) + (P.use_reservoir ? sizeof(T) : 0.0)) +
                           sizeof(T) * (P.n_pump_groups + P.n_potential_groups) + sizeof(C) * P.n_pulse_groups;
         prof_end(PHX_KERNEL_RK4_FUSED, a, pt * (double)N_r * N_c);
         ++launches;
         PHX_CUDA(cudaGetLastError());
-        swap_state_with(0);
+        swap_alt();
     }
 
     void step_rk4() {

@@ -76,6 +76,7 @@ struct StageParams {
     T noise_amp;         // dw * sqrt(dt) of this iteration
     T w_sum;             // right fold of this stage sum's weights
     T dV, four_dV;       // dV, 4 dV
+    T inv_dV;            // 1 / dV, correctly rounded (div_known)
     T gamma_c;
     T noise_scale;       // sqrt(gamma_c / (4 dV)), the scale without reservoir
     // imaginary time (--imagTime): the k-stack sums take the complex step
@@ -156,16 +157,48 @@ __device__ __forceinline__ cx<T> shfl_dn1(cx<T> z) {
 // real (checked on the host), so every reservoir expression below is the
 // reference's complex one with a zero imaginary part carried exactly.
 
-// (one_over_h_bar_s g_c) (-i psi) / dV: the stochastic drift of psi
-template <typename T>
-__device__ __forceinline__ cx<T> noise_drift(const StageParams<T>& P, cx<T> in_wf_mi) {
-    const cx<T> d = smul(P.ohb_gc, in_wf_mi);
-    return mk(rdiv(d.re, P.dV), rdiv(d.im, P.dV));
+// x / y, correctly rounded, where the correctly rounded reciprocal z of y is
+// known beforehand: one multiplication and two fused multiply-adds (Brisebarre,
+// Muller, Raina, "Accelerating correctly rounded floating-point division when
+// the divisor is known in advance", IEEE Trans. Comput. 53(8), 2004).  It holds
+// while the residual does not underflow, in FP32 for |x| > 2^-100; below that
+// the last bit may differ, and an exact zero may change its sign.
+__device__ __forceinline__ float div_known(float x, float y, float z) {
+    const float q = __fmul_rn(x, z);
+    return __fmaf_rn(__fmaf_rn(-q, y, x), z, q);
+}
+__device__ __forceinline__ double div_known(double x, double y, double z) {
+    const double q = __dmul_rn(x, z);
+    return __fma_rn(__fma_rn(-q, y, x), z, q);
 }
 
+// (one_over_h_bar_s g_c) (-i psi) / dV: the stochastic drift of psi
+template <typename T, typename Src>
+__device__ __forceinline__ cx<T> noise_drift(const StageParams<T>& P, const Src& src, cx<T> in_wf_mi) {
+    const cx<T> d = smul(P.ohb_gc, in_wf_mi);
+    return mk(src.over_dV(P, d.re), src.over_dV(P, d.im));
+}
+
+// The pointwise inputs of one point (group g) read from the global planes
+template <typename T>
+struct ScalarGlobalSrc {
+    const StageParams<T>& P;
+    long long idx;
+    __device__ __forceinline__ int n_pump() const { return P.n_pump; }
+    __device__ __forceinline__ int n_pot() const { return P.n_pot; }
+    __device__ __forceinline__ int n_pulse() const { return P.n_pulse; }
+    __device__ __forceinline__ bool noise() const { return P.noise.on != 0; }
+    // real_pot: every potential coefficient is known to be real
+    static __device__ __forceinline__ constexpr bool real_pot() { return false; }
+    static __device__ __forceinline__ T over_dV(const StageParams<T>& S, T x) { return rdiv(x, S.dV); }
+    __device__ __forceinline__ T pump(int g) const { return __ldg(P.pump + idx + g * P.plane); }
+    __device__ __forceinline__ T pot(int g) const { return __ldg(P.pot + idx + g * P.plane); }
+    __device__ __forceinline__ cx<T> pulse(int g) const { return ld1(P.pulse + idx + g * P.plane); }
+};
+
 // Right-hand side of gp_scalar, scalar branch, one grid point.
-template <typename T, bool RES>
-__device__ __forceinline__ void rhs_scalar(const StageParams<T>& P, long long idx, cx<T> in_wf, cx<T> up, cx<T> dn,
+template <typename T, bool RES, typename Src>
+__device__ __forceinline__ void rhs_scalar_src(const StageParams<T>& P, const Src& src, cx<T> in_wf, cx<T> up, cx<T> dn,
                                            cx<T> left, cx<T> right, T in_rv, cx<T>& k_wf, T& k_rv) {
     const cx<T> in_wf_mi = mi(in_wf);
     const T in_psi_norm = abs2(in_wf);
@@ -175,29 +208,33 @@ __device__ __forceinline__ void rhs_scalar(const StageParams<T>& P, long long id
     wf = cadd(wf, smul(rmul(P.ohb_gc, in_psi_norm), in_wf_mi));
     wf = csub(wf, smul(P.half_gamma_c, in_wf));
     if constexpr (RES) {
-        const cx<T> rv = mk(in_rv, (T)0);
-        wf = cadd(wf, cmul(smul(P.ohb_gr, rv), in_wf_mi));
-        wf = cadd(wf, cmul(smul(P.half_R, rv), in_wf));
+        // the reference's complex products with a reservoir of imaginary part
+        // zero, less the products with that zero (only the sign of an exact
+        // zero could tell)
+        wf = cadd(wf, smul(rmul(P.ohb_gr, in_rv), in_wf_mi));
+        wf = cadd(wf, smul(rmul(P.half_R, in_rv), in_wf));
         const T s = -radd(P.gamma_r, rmul(P.R, in_psi_norm));
         T krv = rmul(s, in_rv);
-        for (int g = 0; g < P.n_pump; ++g) krv = radd(krv, rmul(__ldg(P.pump + idx + g * P.plane), P.pump_c[g].re));
+        for (int g = 0; g < src.n_pump(); ++g) krv = radd(krv, rmul(src.pump(g), P.pump_c[g].re));
         k_rv = krv;
     }
-    for (int g = 0; g < P.n_pot; ++g) {
-        const T v = __ldg(P.pot + idx + g * P.plane);
-        const cx<T> pot = smul(v, P.pot_c[g]);
-        wf = cadd(wf, cmul(smul(P.ohb, pot), in_wf_mi));
+    for (int g = 0; g < src.n_pot(); ++g) {
+        const T v = src.pot(g);
+        wf = cadd(wf, src.real_pot() ? smul(rmul(P.ohb, rmul(v, P.pot_c[g].re)), in_wf_mi)
+                                     : cmul(smul(P.ohb, smul(v, P.pot_c[g])), in_wf_mi));
     }
-    for (int g = 0; g < P.n_pulse; ++g) {
-        const cx<T> pulse = ld1(P.pulse + idx + g * P.plane);
-        wf = cadd(wf, cmul(smul(P.ohb, pulse), P.pulse_c[g]));
-    }
-    if (P.noise.on) {
+    for (int g = 0; g < src.n_pulse(); ++g) wf = cadd(wf, cmul(smul(P.ohb, src.pulse(g)), P.pulse_c[g]));
+    if (src.noise()) {
         // stochastic drift (kernel_gp_compute.cuh:82-84, 101-103)
-        wf = csub(wf, noise_drift(P, in_wf_mi));
-        if constexpr (RES) k_rv = radd(k_rv, rdiv(rmul(P.R, in_rv), P.dV));
+        wf = csub(wf, noise_drift(P, src, in_wf_mi));
+        if constexpr (RES) k_rv = radd(k_rv, src.over_dV(P, rmul(P.R, in_rv)));
     }
     k_wf = wf;
+}
+template <typename T, bool RES>
+__device__ __forceinline__ void rhs_scalar(const StageParams<T>& P, long long idx, cx<T> in_wf, cx<T> up, cx<T> dn,
+                                           cx<T> left, cx<T> right, T in_rv, cx<T>& k_wf, T& k_rv) {
+    rhs_scalar_src<T, RES>(P, ScalarGlobalSrc<T>{P, idx}, in_wf, up, dn, left, right, in_rv, k_wf, k_rv);
 }
 
 // dw term of a stage sum at interior point (r, c): w_sum * xi * sqrt((R n0 +

@@ -104,9 +104,10 @@ __device__ __forceinline__ void rhs_tetm_src(const TetmParams<T>& Q, const Src& 
 
     // wavefunction plus
     cx<T> res = smul(Q.ohb_meff, hrp);
-    for (int g = 0; g < P.n_pot; ++g) {
-        const cx<T> pot = smul(src.pot(0, g), P.pot_c[g]);
-        res = cadd(res, cmul(smul(P.ohb, pot), in_wf_plus_mi));
+    for (int g = 0; g < src.n_pot(); ++g) {
+        const T v = src.pot(0, g);
+        res = cadd(res, src.real_pot() ? smul(rmul(P.ohb, rmul(v, P.pot_c[g].re)), in_wf_plus_mi)
+                                       : cmul(smul(P.ohb, smul(v, P.pot_c[g])), in_wf_plus_mi));
     }
     res = cadd(res, smul(rmul(P.ohb_gc, npl), in_wf_plus_mi));
     res = cadd(res, smul(rmul(P.ohb_gr, rvp), in_wf_plus_mi));
@@ -114,19 +115,20 @@ __device__ __forceinline__ void rhs_tetm_src(const TetmParams<T>& Q, const Src& 
     res = csub(res, smul(P.half_gamma_c, wp));
     res = cadd(res, smul(rmul(Q.ohb_gpm, nmi), in_wf_plus_mi));
     res = cadd(res, smul(Q.ohb_dlt, hcp));
-    for (int g = 0; g < P.n_pulse; ++g) res = cadd(res, cmul(smul(P.ohb, src.pulse(0, g)), P.pulse_c[g]));
-    if (P.noise.on) res = csub(res, noise_drift(P, in_wf_plus_mi));
+    for (int g = 0; g < src.n_pulse(); ++g) res = cadd(res, cmul(smul(P.ohb, src.pulse(0, g)), P.pulse_c[g]));
+    if (src.noise()) res = csub(res, noise_drift(P, src, in_wf_plus_mi));
     kwp = res;
     // reservoir plus
     T r = rmul(-radd(P.gamma_r, rmul(P.R, npl)), rvp);
-    for (int g = 0; g < P.n_pump; ++g) r = radd(r, rmul(src.pump(0, g), P.pump_c[g].re));
-    if (P.noise.on) r = radd(r, rdiv(rmul(P.R, rvp), P.dV));
+    for (int g = 0; g < src.n_pump(); ++g) r = radd(r, rmul(src.pump(0, g), P.pump_c[g].re));
+    if (src.noise()) r = radd(r, src.over_dV(P, rmul(P.R, rvp)));
     krp = r;
     // wavefunction minus
     res = smul(Q.ohb_meff, hrm);
-    for (int g = 0; g < P.n_pot; ++g) {
-        const cx<T> pot = smul(src.pot(1, g), P.pot_c[g]);
-        res = cadd(res, cmul(smul(P.ohb, pot), in_wf_minus_mi));
+    for (int g = 0; g < src.n_pot(); ++g) {
+        const T v = src.pot(1, g);
+        res = cadd(res, src.real_pot() ? smul(rmul(P.ohb, rmul(v, P.pot_c[g].re)), in_wf_minus_mi)
+                                       : cmul(smul(P.ohb, smul(v, P.pot_c[g])), in_wf_minus_mi));
     }
     res = cadd(res, smul(rmul(P.ohb_gc, nmi), in_wf_minus_mi));
     res = cadd(res, smul(rmul(P.ohb_gr, rvm), in_wf_minus_mi));
@@ -134,13 +136,13 @@ __device__ __forceinline__ void rhs_tetm_src(const TetmParams<T>& Q, const Src& 
     res = csub(res, smul(P.half_gamma_c, wm));
     res = cadd(res, smul(rmul(Q.ohb_gpm, npl), in_wf_minus_mi));
     res = cadd(res, smul(Q.ohb_dlt, hcm));
-    for (int g = 0; g < P.n_pulse; ++g) res = cadd(res, cmul(smul(P.ohb, src.pulse(1, g)), P.pulse_c[g]));
-    if (P.noise.on) res = csub(res, noise_drift(P, in_wf_minus_mi));
+    for (int g = 0; g < src.n_pulse(); ++g) res = cadd(res, cmul(smul(P.ohb, src.pulse(1, g)), P.pulse_c[g]));
+    if (src.noise()) res = csub(res, noise_drift(P, src, in_wf_minus_mi));
     kwm = res;
     // reservoir minus
     r = rmul(-radd(P.gamma_r, rmul(P.R, nmi)), rvm);
-    for (int g = 0; g < P.n_pump; ++g) r = radd(r, rmul(src.pump(1, g), P.pump_c[g].re));
-    if (P.noise.on) r = radd(r, rdiv(rmul(P.R, rvm), P.dV));
+    for (int g = 0; g < src.n_pump(); ++g) r = radd(r, rmul(src.pump(1, g), P.pump_c[g].re));
+    if (src.noise()) r = radd(r, src.over_dV(P, rmul(P.R, rvm)));
     krm = r;
 }
 
@@ -150,6 +152,12 @@ template <typename T>
 struct TetmGlobalSrc {
     const TetmParams<T>& Q;
     long long idx;
+    __device__ __forceinline__ int n_pump() const { return Q.p.n_pump; }
+    __device__ __forceinline__ int n_pot() const { return Q.p.n_pot; }
+    __device__ __forceinline__ int n_pulse() const { return Q.p.n_pulse; }
+    __device__ __forceinline__ bool noise() const { return Q.p.noise.on != 0; }
+    static __device__ __forceinline__ constexpr bool real_pot() { return false; }
+    static __device__ __forceinline__ T over_dV(const StageParams<T>& S, T x) { return rdiv(x, S.dV); }
     __device__ __forceinline__ T pump(int c, int g) const { return __ldg((c ? Q.pump : Q.p.pump) + idx + g * Q.p.plane); }
     __device__ __forceinline__ T pot(int c, int g) const { return __ldg((c ? Q.pot : Q.p.pot) + idx + g * Q.p.plane); }
     __device__ __forceinline__ cx<T> pulse(int c, int g) const { return ld1((c ? Q.pulse : Q.p.pulse) + idx + g * Q.p.plane); }

@@ -58,6 +58,12 @@ struct TetmTileSrc {
     long long idx;
     const T* in;  // [pump+, pump-, pot+, pot-][NR] at this point: in + q
     int NR;
+    __device__ __forceinline__ int n_pump() const { return Q.p.n_pump; }
+    __device__ __forceinline__ int n_pot() const { return Q.p.n_pot; }
+    __device__ __forceinline__ int n_pulse() const { return Q.p.n_pulse; }
+    __device__ __forceinline__ bool noise() const { return Q.p.noise.on != 0; }
+    static __device__ __forceinline__ constexpr bool real_pot() { return false; }
+    static __device__ __forceinline__ T over_dV(const StageParams<T>& S, T x) { return rdiv(x, S.dV); }
     __device__ __forceinline__ T pump(int c, int g) const {
         return g == 0 ? in[c * NR] : __ldg((c ? Q.pump : Q.p.pump) + idx + g * Q.p.plane);
     }

@@ -67,3 +67,52 @@ def test_fma_arithmetic(require_gpu, monkeypatch, res, pot, temporal):
     b = run(114, 70, "f32", True, True, 4, monkeypatch, res, True, pot, temporal, fma=True)
     for x, y in zip(a, b):
         np.testing.assert_array_equal(x, y)
+
+
+def general(n_c, n_r, dtype, px, py, monkeypatch, staged, tetm=False, pumps=1, pot=1, pulse=0, dw=0.0, iters=4):
+    monkeypatch.setenv("PHX_TETM_FUSED", "0" if staged else "1")
+    monkeypatch.setenv("PHX_GENERAL_FUSED", "0" if staged else "1")
+    T = pb.Temporal
+    rng = np.random.default_rng([n_c, n_r, 3])
+    sp = pb.SystemParameters(N_c=n_c, N_r=n_r, L_x=0.3 * n_c, L_y=0.2 * n_r, h_bar_s=0.6582, m_eff=0.5, gamma_c=0.2,
+                             gamma_r=0.3, g_c=0.05, g_r=0.08, R=0.04, g_pm=-0.01, delta_LT=0.3, use_twin_mode=tetm,
+                             periodic_boundary_x=px, periodic_boundary_y=py, dtype=dtype, dt=0.002, t_max=1e12,
+                             fft_every=1e12, pump_temporal=[T(), T("cos", 0.004, 0.01, 200.0)][:pumps],
+                             potential_temporal=[T("gauss", 0.004, 0.01, 1.0)][:pot],
+                             pulse_temporal=[T("iexp", 0.004, 0.01, 50.0)][:pulse], stochastic_amplitude=dw, random_seed=11)
+    comps = ("plus", "minus") if tetm else ("plus",)
+    with pb.Solver(sp) as s:
+        for c in comps:
+            z = lambda: rng.standard_normal((n_r, n_c)) + 1j * rng.standard_normal((n_r, n_c))  # noqa: E731
+            s.set_field("psi_" + c, z())
+            s.set_field("n_" + c, rng.random((n_r, n_c)))
+            for g in range(pumps):
+                s.set_field("pump_" + c, 3.0 * rng.random((n_r, n_c)), g)
+            for g in range(pot):
+                s.set_field("potential_" + c, 0.3 * rng.standard_normal((n_r, n_c)), g)
+            for g in range(pulse):
+                s.set_field("pulse_" + c, z(), g)
+        info = s.run(iters)
+        assert staged == (info.kernel_launches >= 4 * iters)
+        return [s.get_field(f + c) for c in comps for f in ("psi_", "n_")]
+
+
+# what a step's template parameters select, on grids around one and two strips;
+# the scalar model without any of them is the plain iteration above
+INPUTS = [(1, 1, 0, 0.02), (1, 0, 0, 0.02), (1, 1, 1, 0.0), (1, 0, 1, 0.02), (2, 1, 1, 0.0), (2, 0, 0, 0.02)]
+
+
+@pytest.mark.parametrize("tetm,dtype,pumps,pot,pulse,dw",
+                         [(False, d) + i for d in ("f32", "f64") for i in INPUTS] +
+                         [(True, d) + i for d in ("f32", "f64") for i in INPUTS + [(1, 1, 0, 0.0)]])
+def test_general_and_spinor_iterations(require_gpu, monkeypatch, tetm, dtype, pumps, pot, pulse, dw):
+    sizes = [(8, 8, True, True), (56, 13, True, False), (114, 61, False, True)]
+    if dw > 0 or dtype == "f64":  # below 280000 points these run the tile kernels: the same widths, taller
+        sizes = [(8, 35001, True, True), (56, 5003, True, False), (114, 2461, False, True)]
+    if dtype == "f64":
+        sizes.append((57, 4913, False, False))
+    for n_c, n_r, px, py in sizes:
+        want = general(n_c, n_r, dtype, px, py, monkeypatch, True, tetm, pumps, pot, pulse, dw)
+        got = general(n_c, n_r, dtype, px, py, monkeypatch, False, tetm, pumps, pot, pulse, dw)
+        for x, y in zip(got, want):
+            np.testing.assert_array_equal(x, y, err_msg=f"{n_c} x {n_r}")
