@@ -317,8 +317,8 @@ PHX_API phx_status phx_get_field_device(phx_handle* h, int32_t field, int32_t gr
  * right-hand side as in gp_scalar (include/kernel/kernel_gp_compute.cuh:86-98):
  * dL/dP through the reservoir's gain P c_P(t), dL/dV through
  * (c_V(t) / hbar) V (-i psi).
- * The recompute of the next segment runs on a second stream that the call
- * creates, beside the current segment's gradient sweep, so two segments'
+ * The recompute of the next segment runs on a second stream of the handle,
+ * beside the current segment's gradient sweep, so two segments'
  * states and stage values are held at once; the call returns after both
  * streams' work is done.  All arrays are contiguous N_r x N_c device arrays in
  * the build precision; the adjoint of a complex value u + iv is

@@ -78,7 +78,7 @@ def build_host(force: bool = False, verbose: bool = False) -> None:
 
 
 UNITS = ["phx_runtime.cu", "phx_noalloc.cu", "phx_batch.cu", "phx_march.cu",
-         "phx_march_general.cu"]
+         "phx_march_general.cu", "phx_adjoint_march.cu"]
 OBJ_DIR = os.path.join(PKG, "_build")
 
 

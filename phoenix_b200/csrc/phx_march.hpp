@@ -6,6 +6,7 @@
 #include <map>
 #include <vector>
 
+#include "phx_adjoint.cuh"
 #include "phx_rt.hpp"
 #include "phx_stage_tetm.cuh"
 
@@ -65,6 +66,25 @@ private:
     int plan_rows_ = 0;
 };
 
+// The adjoint's four vector-Jacobian stages of one iteration
+// (phx_adjoint_march.cuh, compiled in phx_adjoint_march.cu); planes as
+// MarchLauncher::fits.
+template <typename T>
+class AdjMarch {
+public:
+    // whether the kernel wraps around the grid itself, so that neither the stage
+    // values nor lam' need periodic images
+    static bool wraps(int N_c) { return N_c % 2 == 0; }
+    void launch(const AdjFusedParams<T>& Q, int sm_count, cudaStream_t stream, bool pdl);
+
+private:
+    std::map<const void*, int> per_sm_;  // CTAs per SM of the kernel variants used so far
+    std::array<int, 4> plan_{};          // grid, CTAs per SM and SMs of the last row segmentation
+    int plan_rows_ = 0;
+};
+
+extern template class AdjMarch<float>;
+extern template class AdjMarch<double>;
 extern template class MarchGeneral<float>;
 extern template class MarchGeneral<double>;
 extern template class MarchBatch<float>;

@@ -45,11 +45,17 @@ struct Error {
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    bool owned = true;  // false: a part of another buffer (view)
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() {
-        if (p) cudaFree(p);
+        if (p && owned) cudaFree(p);
+    }
+    void view(void* part, size_t n) {
+        p = part;
+        bytes = n;
+        owned = false;
     }
     void alloc(size_t n, cudaStream_t s) {
         if (p) cudaFree(p);

@@ -851,11 +851,12 @@ struct Engine final : EngineBase {
     }
     // ---- marching warps (phx_step_march.cuh)
     MarchLauncher<T> march;
-    void go_march(const FusedParams<T>& F, bool res, bool fma) {
+    void go_march(const FusedParams<T>& F, bool res, bool fma, bool store = false) {
         if (!sm_count) PHX_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, P.device));
         MarchOptions o;
         o.res = res;
         o.fma = fma;
+        o.store = store;
         o.pdl = pdl_on();
         march.launch(F, o, sm_count, stream);
     }
@@ -2008,6 +2009,24 @@ struct Engine final : EngineBase {
     std::vector<std::unique_ptr<DevBuf>> st_psi, st_n;    // Y2..Y4 of every iteration of a segment
     std::vector<std::unique_ptr<DevBuf>> sg_psi2, sg_n2, st_psi2, st_n2;  // the second set (overlapped recompute)
     DevBuf lam_psi[2], lam_n[2], yb_psi[2], yb_n[2], la_psi, la_n, pbar, vbar;
+    DevBuf scratch_psi, scratch_n;
+    // the second stream of the backward and its events, kept for the next call
+    struct Overlap {
+        cudaStream_t s2 = nullptr;
+        cudaEvent_t start = nullptr, rec_done[2] = {nullptr, nullptr}, vjp_done[2] = {nullptr, nullptr};
+        void create() {
+            if (!s2) PHX_CUDA(cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking));
+            for (cudaEvent_t* e : {&start, &rec_done[0], &rec_done[1], &vjp_done[0], &vjp_done[1]})
+                if (!*e) PHX_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        }
+        ~Overlap() {
+            if (s2) (void)cudaStreamSynchronize(s2);
+            for (cudaEvent_t e : {start, rec_done[0], rec_done[1], vjp_done[0], vjp_done[1]})
+                if (e) (void)cudaEventDestroy(e);
+            if (s2) (void)cudaStreamDestroy(s2);
+        }
+    } ov;
+    AdjMarch<T> adj_march;
     int64_t adj_T = 0, adj_every = 0;
     T adj_dt = 0;
     bool adj_ready = false;
@@ -2033,10 +2052,17 @@ struct Engine final : EngineBase {
     void plane_copy(DevBuf& dst, const DevBuf& src) {
         PHX_CUDA(cudaMemcpyAsync(dst.p, src.p, src.bytes, cudaMemcpyDeviceToDevice, stream));
     }
+    // at least n planes in v, the missing ones out of one allocation (some 200
+    // planes for 200 iterations: one cudaMalloc each took 100 ms)
+    std::vector<std::unique_ptr<DevBuf>> adj_slabs;
     void ensure_planes(std::vector<std::unique_ptr<DevBuf>>& v, size_t n, size_t bytes) {
-        while (v.size() < n) {
+        if (v.size() >= n) return;
+        const size_t more = n - v.size(), step = (bytes + 255) / 256 * 256;
+        adj_slabs.emplace_back(new DevBuf());
+        adj_slabs.back()->alloc(step * more, stream);
+        for (size_t i = 0; i < more; ++i) {
             v.emplace_back(new DevBuf());
-            v.back()->alloc(bytes, stream);
+            v.back()->view(static_cast<char*>(adj_slabs.back()->p) + i * step, bytes);
         }
     }
     void adjoint_forward(int64_t iterations, int64_t every) override {
@@ -2096,8 +2122,8 @@ struct Engine final : EngineBase {
                 launch<kRk4Last>(S, wire);
         }
     }
-    // storing variants of the non-TMA one-kernel shapes (go_fused's cases 0-3);
-    // false when the tuned shape is not one of them
+    // storing variants of the non-TMA one-kernel shapes (go_fused's cases 0-3
+    // and 8); false when the tuned shape is not one of them
     template <bool RES, int TW, int TH, int NT>
     void go_fused_shape_store(const FusedParams<T>& F) {
         dim3 grid((unsigned)((N_c + TW - 1) / TW), (unsigned)((N_r + TH - 1) / TH));
@@ -2116,6 +2142,10 @@ struct Engine final : EngineBase {
                     go_fused_shape_store<RES, 64, 32, 512>(F);
                 else
                     go_fused_shape_store<RES, 32, 24, 384>(F);
+                return true;
+            case 8:
+                if (!MarchLauncher<T>::fits(plane)) return false;
+                go_march(F, RES, false, true);
                 return true;
             default: return false;
         }
@@ -2184,6 +2214,7 @@ struct Engine final : EngineBase {
         F.n1 = on ? rplane(*on) : nullptr;
         F.pump = P.n_pump_groups ? rplane(pump[0]) : nullptr;
         F.pot = P.n_potential_groups ? rplane(pot[0]) : nullptr;
+        F.st_images = !(adj_fused && MarchLauncher<T>::fits(plane) && AdjMarch<T>::wraps(N_c));
         for (int s = 0; s < 3; ++s) {
             F.st_psi[s] = cplane(*sp[s]);
             F.st_n[s] = sn[s] ? rplane(*sn[s]) : nullptr;
@@ -2266,9 +2297,9 @@ struct Engine final : EngineBase {
         PHX_CUDA(cudaGetLastError());
         const T saved_dt = dt;
         dt = adj_dt;
-        DevBuf scratch_psi, scratch_n;  // the recomputed state after a segment's last iteration is not needed
-        scratch_psi.alloc(cb, stream);
-        if (res) scratch_n.alloc(rb, stream);
+        // the recomputed state after a segment's last iteration is not needed
+        if (!scratch_psi.p) scratch_psi.alloc(cb, stream);
+        if (res && !scratch_n.p) scratch_n.alloc(rb, stream);
         const T bw[4] = {(T)(1.0 / 6.0), (T)(1.0 / 3.0), (T)(1.0 / 3.0), (T)(1.0 / 6.0)};
         const T aw[3] = {(T)0.5, (T)0.5, (T)1.0};
         const T cw[4] = {(T)0.0, (T)0.5, (T)0.5, (T)1.0};
@@ -2278,21 +2309,16 @@ struct Engine final : EngineBase {
         // overlapped with the sweep of the segment before; events order a set's
         // reuse after the sweep that read it.
         const bool overlap = adj_fused;
-        struct Overlap {
-            cudaStream_t s2 = nullptr;
-            cudaEvent_t start = nullptr, rec_done[2] = {nullptr, nullptr}, vjp_done[2] = {nullptr, nullptr};
-            ~Overlap() {
-                if (s2) (void)cudaStreamSynchronize(s2);
-                for (cudaEvent_t e : {start, rec_done[0], rec_done[1], vjp_done[0], vjp_done[1]})
-                    if (e) (void)cudaEventDestroy(e);
-                if (s2) (void)cudaStreamDestroy(s2);
-            }
-        } ov;
         bool vjp_used[2] = {false, false};
+        // an error that leaves this call early still waits for the second stream
+        struct Join {
+            Overlap& o;
+            ~Join() {
+                if (o.s2) (void)cudaStreamSynchronize(o.s2);
+            }
+        } join{ov};
         if (overlap) {
-            PHX_CUDA(cudaStreamCreateWithFlags(&ov.s2, cudaStreamNonBlocking));
-            for (cudaEvent_t* e : {&ov.start, &ov.rec_done[0], &ov.rec_done[1], &ov.vjp_done[0], &ov.vjp_done[1]})
-                PHX_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+            ov.create();
             PHX_CUDA(cudaEventRecord(ov.start, stream));
             PHX_CUDA(cudaStreamWaitEvent(ov.s2, ov.start, 0));
         }
@@ -2384,6 +2410,7 @@ struct Engine final : EngineBase {
                     Q.res = res;
                     cudaEvent_t a = nullptr;
                     prof_begin(a);
+                    if (!sm_count) PHX_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, P.device));
                     auto go_adj = [&](auto tw, auto th, auto nt, auto minb) {
                         constexpr int TW = decltype(tw)::value, TH = decltype(th)::value, NT = decltype(nt)::value;
                         constexpr int MINB = decltype(minb)::value;
@@ -2391,7 +2418,9 @@ struct Engine final : EngineBase {
                         adj_fused_kernel<T, TW, TH, NT, MINB><<<grid, NT, 0, stream>>>(Q);
                     };
                     using std::integral_constant;
-                    if constexpr (sizeof(T) == 4)  // 64 x 16 tiles, 16 warps, two CTAs per SM
+                    if (MarchLauncher<T>::fits(plane))
+                        adj_march.launch(Q, sm_count, stream, pdl_on());
+                    else if constexpr (sizeof(T) == 4)  // 64 x 16 tiles, 16 warps, two CTAs per SM
                         go_adj(integral_constant<int, 64>{}, integral_constant<int, 16>{}, integral_constant<int, 512>{},
                                integral_constant<int, 2>{});
                     else

@@ -107,8 +107,8 @@ __device__ __forceinline__ void ring_two(const unsigned char* p, double* v) {
 // POT: the potential's terms are evaluated (an absent plane counts as zero).
 // UNIT: every temporal coefficient is exactly 1 (constant envelopes); the
 // products with it, which change nothing, are left out.  STORE: also write
-// the stage values Y2..Y4 of the stored points (with periodic images), which
-// the adjoint's backward sweep reads.  Plane indices are 32-bit (the host
+// the stage values Y2..Y4 of the stored points (with periodic images where
+// P.st_images), which the adjoint's backward sweep reads.  Plane indices are 32-bit (the host
 // takes this kernel for planes of fewer than 2^31 points only).
 template <typename T, bool RES, bool POT, bool UNIT, bool FMA, bool STORE>
 __device__ __forceinline__ void march_segment(const FusedParams<T>& P, int strip, int R0, int R1, unsigned char* ring) {
@@ -258,7 +258,8 @@ __device__ __forceinline__ void march_segment(const FusedParams<T>& P, int strip
         }
         const int row = R0 - 4 + k - s;
         if constexpr (STORE && s < 3) {
-            if (row >= R0 && row < R1) put(P.st_psi[own], P.st_n[own], row, o, on);
+            if (store_lane && row >= R0 && row < R1) put_at(P.st_psi[own], P.st_n[own], row * pitch + c, o, on);
+            if (P.st_images && row >= R0 && row < R1) put(P.st_psi[own], P.st_n[own], row, o, on);
         }
         if constexpr (s == 3) put(P.psi1, P.n1, row, o, on);
     };
