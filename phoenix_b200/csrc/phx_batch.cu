@@ -269,7 +269,27 @@ struct BatchEngine final : BatchBase {
         const int smem = TmaLayout<T, SH::TW[S], SH::TH[S]>::total;
         kernel_of<S>()<<<blocks[S], SH::NT[S], smem, stream>>>(B);
     }
+    // the marching warps leave no periodic images behind (unless march.images());
+    // the tile kernels read them
+    bool images_ok = true;
+    void fill_rings(int plane) {
+        for (auto& ip : inst) {
+            Instance& I = *ip;
+            ring_fill_kernel<C><<<64, 256, 0, stream>>>(I.cplane(I.psi[plane]), I.P.N_r, I.P.N_c, I.pitch, G, I.P.periodic_x,
+                                                        I.P.periodic_y);
+            if (res)
+                ring_fill_kernel<T><<<64, 256, 0, stream>>>(I.rplane(I.n[plane]), I.P.N_r, I.P.N_c, I.pitch, G, I.P.periodic_x,
+                                                            I.P.periodic_y);
+        }
+        PHX_CUDA(cudaGetLastError());
+    }
+    void prepare_rings(int sh, int dir) {
+        const bool reads = sh != kBatchMarch || march.images();
+        if (reads && !images_ok) fill_rings(dir);
+        images_ok = reads;
+    }
     void launch(int sh, int dir) {
+        prepare_rings(sh, dir);
         switch (sh) {
             case 0: go<0>(dir); break;
             case 1: go<1>(dir); break;
@@ -299,6 +319,7 @@ struct BatchEngine final : BatchBase {
     void tune_iteration() {
         const int sh = tune_step % kBatchShapes;
         cudaEvent_t a = event(), b = event();
+        prepare_rings(sh, cur);  // not charged to the shape that is timed
         PHX_CUDA(cudaEventRecord(a, stream));
         launch(sh, cur);
         PHX_CUDA(cudaEventRecord(b, stream));

@@ -27,29 +27,38 @@ void MarchLauncher<T>::launch(const FusedParams<T>& F, const MarchOptions& o, in
     // the variant with temporal coefficients always takes the potential's terms
     const bool pot = F.pot != nullptr || !unit;
     K kern = nullptr;
-    auto pick = [&](auto res, auto fma, auto store) {
-        constexpr bool R = decltype(res)::value, M = decltype(fma)::value, S = decltype(store)::value;
-        kern = !pot ? (K)rk4_march_kernel<T, R, false, true, M, S, MINB>
-                    : (unit ? (K)rk4_march_kernel<T, R, true, true, M, S, MINB> : (K)rk4_march_kernel<T, R, true, false, M, S, MINB>);
-    };
     using std::false_type;
     using std::true_type;
+    auto pick = [&](auto res, auto fma, auto img) {
+        constexpr bool R = decltype(res)::value, M = decltype(fma)::value, I = decltype(img)::value;
+        kern = !pot ? (K)rk4_march_kernel<T, R, false, true, M, false, I, MINB>
+                    : (unit ? (K)rk4_march_kernel<T, R, true, true, M, false, I, MINB>
+                            : (K)rk4_march_kernel<T, R, true, false, M, false, I, MINB>);
+    };
+    auto pick_store = [&](auto res, auto img) {
+        constexpr bool R = decltype(res)::value, I = decltype(img)::value;
+        kern = pot ? (K)rk4_march_kernel<T, R, true, true, false, true, I, MINB>
+                   : (K)rk4_march_kernel<T, R, false, true, false, true, I, MINB>;
+    };
     if (o.store) {
-        if (o.fma || !unit) fail(PHX_ERR_UNSUPPORTED, "stage values are stored in the bit-exact arithmetic with constant envelopes");
-        if (o.res)
-            kern = pot ? (K)rk4_march_kernel<T, true, true, true, false, true, MINB> : (K)rk4_march_kernel<T, true, false, true, false, true, MINB>;
-        else
-            kern = pot ? (K)rk4_march_kernel<T, false, true, true, false, true, MINB> : (K)rk4_march_kernel<T, false, false, true, false, true, MINB>;
+        if (!unit) fail(PHX_ERR_UNSUPPORTED, "stage values are stored with constant envelopes");
+        if (o.res) o.img ? pick_store(true_type{}, true_type{}) : pick_store(true_type{}, false_type{});
+        else o.img ? pick_store(false_type{}, true_type{}) : pick_store(false_type{}, false_type{});
     } else if (o.fma) {
         if constexpr (sizeof(T) == 4) {
             if (o.res) pick(true_type{}, true_type{}, false_type{});
             else pick(false_type{}, true_type{}, false_type{});
         }
+    } else if (o.img) {
+        if constexpr (sizeof(T) == 8) {  // odd numbers of columns are FP64's
+            if (o.res) pick(true_type{}, false_type{}, true_type{});
+            else pick(false_type{}, false_type{}, true_type{});
+        }
     } else {
         if (o.res) pick(true_type{}, false_type{}, false_type{});
         else pick(false_type{}, false_type{}, false_type{});
     }
-    if (!kern) fail(PHX_ERR_UNSUPPORTED, "the fused multiply-add arithmetic is FP32 only");
+    if (!kern) fail(PHX_ERR_UNSUPPORTED, "no marching variant for these options");
     int& per_sm = per_sm_[reinterpret_cast<const void*>(kern)];
     if (!per_sm) per_sm = march_occupancy(kern, Lay::bytes);
     MarchParams<T> Q;
@@ -78,17 +87,22 @@ void MarchBatch<T>::build(const std::vector<FusedParams<T>>& f, bool res, bool f
         max_rows = std::max(max_rows, f[2 * i].N_r);
     }
     K kern = nullptr;
-    auto pick = [&](auto m) {
-        constexpr bool M = decltype(m)::value;
+    auto pick = [&](auto m, auto img) {
+        constexpr bool M = decltype(m)::value, I = decltype(img)::value;
         if (res)
-            kern = pot ? (K)rk4_march_batch_kernel<T, true, true, M, MINB> : (K)rk4_march_batch_kernel<T, true, false, M, MINB>;
+            kern = pot ? (K)rk4_march_batch_kernel<T, true, true, M, I, MINB> : (K)rk4_march_batch_kernel<T, true, false, M, I, MINB>;
         else
-            kern = pot ? (K)rk4_march_batch_kernel<T, false, true, M, MINB> : (K)rk4_march_batch_kernel<T, false, false, M, MINB>;
+            kern = pot ? (K)rk4_march_batch_kernel<T, false, true, M, I, MINB>
+                       : (K)rk4_march_batch_kernel<T, false, false, M, I, MINB>;
     };
+    images_ = false;
+    for (int i = 0; i < n; ++i) images_ = images_ || march_needs_images(f[2 * i].N_c, f[2 * i].img_x);
     if constexpr (sizeof(T) == 4) {
-        if (fma) pick(std::true_type{});
+        if (fma) pick(std::true_type{}, std::false_type{});
+    } else {
+        if (images_) pick(std::false_type{}, std::true_type{});
     }
-    if (!kern) pick(std::false_type{});
+    if (!kern) pick(std::false_type{}, std::false_type{});
     const int per_sm = march_occupancy(kern, MarchLayout<T>::bytes);
     auto strips = [&](int i) { return (f[2 * i].N_c + kMarchOut - 1) / kMarchOut; };
     const int L = march_seg_rows<T>(

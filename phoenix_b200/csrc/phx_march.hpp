@@ -12,10 +12,15 @@
 
 namespace phx {
 
+// whether the marching iterations read and write the periodic images in the
+// planes' rings: only where column pairs cannot wrap around the grid
+inline bool march_needs_images(int N_c, int periodic_x) { return periodic_x && N_c % 2 != 0; }
+
 struct MarchOptions {
     bool res = true;     // reservoir
     bool fma = false;    // fused multiply-add arithmetic (FP32)
     bool store = false;  // also write the stage values (FusedParams::st_psi / st_n)
+    bool img = false;    // read and write periodic images (march_needs_images, or another reader needs them)
     bool pdl = true;     // programmatic stream serialization
 };
 
@@ -40,8 +45,11 @@ public:
     // f: two directions per instance (constant envelopes); waits for the copies
     void build(const std::vector<FusedParams<T>>& f, bool res, bool fma, int sm_count, cudaStream_t stream);
     void launch(int dir, cudaStream_t stream) const;
+    // whether the launches read and write periodic images (march_needs_images)
+    bool images() const { return images_; }
 
 private:
+    bool images_ = false;
     DevBuf f_, items_;
     const void* kern_ = nullptr;
     int n_items_ = 0;

@@ -12,7 +12,7 @@ using GeneralKernel = void (*)(MarchGeneralParams<T, COMPS>);
 
 struct Variant {
     int np, nv, nq;
-    bool noise;
+    bool noise, img;
 };
 
 // kernel and shared memory of a variant; a null kernel when there is none
@@ -20,7 +20,10 @@ template <typename T, int COMPS, int NP, int NV, int NQ, bool NOISE>
 void take(const Variant& v, GeneralKernel<T, COMPS>& k, int& bytes) {
     if (v.np != NP || v.nv != NV || v.nq != NQ || v.noise != NOISE) return;
     constexpr int MINB = COMPS == 1 && sizeof(T) == 4 ? 3 : 2;
-    k = rk4_march_general_kernel<T, COMPS, true, NP, NV, NQ, NOISE, true, MINB>;
+    k = rk4_march_general_kernel<T, COMPS, true, NP, NV, NQ, NOISE, true, false, MINB>;
+    if constexpr (sizeof(T) == 8) {  // odd numbers of columns are FP64's
+        if (v.img) k = rk4_march_general_kernel<T, COMPS, true, NP, NV, NQ, NOISE, true, true, MINB>;
+    }
     bytes = MarchGeneralLayout<T, COMPS, true, NP, NV, NQ, NOISE>::bytes;
 }
 template <typename T, int COMPS, int NP, int NV, int NQ>
@@ -44,7 +47,7 @@ template <int COMPS>
 bool MarchGeneral<T>::launch_comps(const TetmParams<T> (&st)[4], const cx<T>* const* psi0, const T* const* n0,
                                    cx<T>* const* psi1, T* const* n1, int sm_count, cudaStream_t stream, bool pdl) {
     const StageParams<T>& P = st[0].p;
-    const Variant v{P.n_pump, P.n_pot, P.n_pulse, P.noise.on != 0};
+    const Variant v{P.n_pump, P.n_pot, P.n_pulse, P.noise.on != 0, march_needs_images(P.N_c, P.img_x)};
     GeneralKernel<T, COMPS> kern = nullptr;
     int bytes = 0;
     take_rest<T, COMPS, 1>(v, kern, bytes);

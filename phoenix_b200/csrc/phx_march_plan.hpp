@@ -9,29 +9,29 @@
 
 namespace phx {
 
-// Rows per segment.  A segment of L rows costs about L + 3 full steps (its
-// first rows run through some stages only), and an SM with w CTAs takes
-// cost[w] per step of all of them (measured at 1024^2; one CTA leaves its
-// schedulers waiting on one warp's latencies).  More CTAs than fit at once
-// follow one another without a common end, hence the fractional rounds.
+// Rows per segment.  A segment of L rows costs about L + extra full steps (its
+// first rows run through some stages only; four stages: 3), and an SM with w
+// CTAs takes cost(w) per step of all of them (measured at 1024^2; one CTA
+// leaves its schedulers waiting on one warp's latencies).  More CTAs than fit
+// at once run in rounds.  4096^2 FP32: 184 us at 64 rows (estimate 189), 196 at
+// 32 (199).
 template <typename T>
-double march_cost(int L, long long items, int per_sm, int sm_count) {
-    const double cost32[4] = {0.0, 0.61, 0.86, 1.2}, cost64[3] = {0.0, 0.94, 1.55};
+double march_cost(int L, long long items, int per_sm, int sm_count, double extra) {
+    const double cost32[4] = {0.0, 0.47, 0.74, 1.05}, cost64[3] = {0.0, 0.92, 1.52};
     auto cost = [&](int w) {
         if (sizeof(T) == 4) return w <= 3 ? cost32[w] : cost32[3] * w / 3;
         return w <= 2 ? cost64[w] : cost64[2] * w / 2;
     };
     const long long ctas = (items + kMarchWarps - 1) / kMarchWarps, w = (ctas + sm_count - 1) / sm_count;
-    return (L + 3.0) *
-           (w <= per_sm ? cost((int)w) : ((double)ctas / ((double)per_sm * sm_count) + 0.3) * cost(per_sm));
+    return (L + extra) * ((double)(w / per_sm) * cost(per_sm) + cost((int)(w % per_sm)));
 }
 // the cheapest segment length of at most max_rows, items(L) segments in all
 template <typename T, typename Items>
-int march_seg_rows(int max_rows, const Items& items, int per_sm, int sm_count) {
+int march_seg_rows(int max_rows, const Items& items, int per_sm, int sm_count, double extra = 3.0) {
     int best_L = max_rows;
     double best = -1.0;
     for (int L = std::min(max_rows, 2); L <= std::min(max_rows, 256); ++L) {
-        const double t = march_cost<T>(L, items(L), per_sm, sm_count);
+        const double t = march_cost<T>(L, items(L), per_sm, sm_count, extra);
         if (best < 0.0 || t < best) best = t, best_L = L;
     }
     return best_L;

@@ -851,12 +851,34 @@ struct Engine final : EngineBase {
     }
     // ---- marching warps (phx_step_march.cuh)
     MarchLauncher<T> march;
+    // The marching iterations wrap around the grid themselves and leave no
+    // periodic images behind (march_needs_images aside); every other kernel
+    // reads them, so the rings are filled again before one runs.
+    bool images_ok = true;
+    void need_images() {
+        if (!images_ok && (P.periodic_x || P.periodic_y))
+            for (int q = 0; q < comps; ++q) {
+                ring_fill_kernel<C><<<64, 256, 0, stream>>>(cplane(psi[q]), N_r, N_c, pitch, G, P.periodic_x, P.periodic_y);
+                ring_fill_kernel<T><<<64, 256, 0, stream>>>(rplane(nres[q]), N_r, N_c, pitch, G, P.periodic_x, P.periodic_y);
+                launches += 2;
+            }
+        PHX_CUDA(cudaGetLastError());
+        images_ok = true;
+    }
+    // the adjoint's planes need images where its sweep does not wrap
+    bool adj_images() const { return !(adj_fused && MarchLauncher<T>::fits(plane) && AdjMarch<T>::wraps(N_c)); }
     void go_march(const FusedParams<T>& F, bool res, bool fma, bool store = false) {
+        const bool img = march_needs_images(N_c, P.periodic_x) || (store && adj_images());
+        if (!store) {
+            if (img) need_images();
+            images_ok = img;
+        }
         if (!sm_count) PHX_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, P.device));
         MarchOptions o;
         o.res = res;
         o.fma = fma;
         o.store = store;
+        o.img = img;
         o.pdl = pdl_on();
         march.launch(F, o, sm_count, stream);
     }
@@ -874,6 +896,7 @@ struct Engine final : EngineBase {
     template <bool RES, bool FMA = false>
     void go_fused(const FusedParams<T>& F) {
         constexpr bool f32 = sizeof(T) == 4;
+        if (cur_shape() - kFusedShape != 8 || !MarchLauncher<T>::fits(plane)) need_images();
         switch (cur_shape() - kFusedShape) {
             case 4: go_tma<RES, 32, f32 ? 32 : 16, 256, 1, FMA>(F); return;
             // 12 warps per CTA, two CTAs per SM: registers capped at 85
@@ -992,7 +1015,14 @@ struct Engine final : EngineBase {
             p1[q] = cplane(psi_alt[q]);
             n1[q] = rplane(n_alt[q]);
         }
-        return march_general.launch(st, comps, P.use_reservoir != 0, p0, n0, p1, n1, sm_count, stream, pdl_on());
+        const bool img = march_needs_images(N_c, P.periodic_x);
+        if (img) need_images();
+        const bool done = march_general.launch(st, comps, P.use_reservoir != 0, p0, n0, p1, n1, sm_count, stream, pdl_on());
+        if (done)
+            images_ok = img;
+        else
+            need_images();
+        return done;
     }
 
     // ---- TE/TM: the whole iteration in one kernel (phx_step_tetm_fused.cuh);
@@ -1134,6 +1164,7 @@ struct Engine final : EngineBase {
             return;
         }
         if (is_fused(cur_shape()) && step_rk4_fused()) return;
+        need_images();
         const T cw[4] = {(T)0.0, (T)0.5, (T)0.5, (T)1.0};
         const T aw[3] = {(T)0.5, (T)0.5, (T)1.0};
         const T bw[4] = {(T)(1.0 / 6.0), (T)(1.0 / 3.0), (T)(1.0 / 3.0), (T)(1.0 / 6.0)};
@@ -1847,6 +1878,8 @@ struct Engine final : EngineBase {
             t = t + dt;
             cudaEvent_t ta = nullptr, tb = nullptr;
             if (shape < 0) {
+                // a candidate is not charged for the images that the marching one left out
+                if (is_fused(cur_shape()) && cur_shape() != kFusedShape + 8) need_images();
                 ta = get_event();
                 PHX_CUDA(cudaEventRecord(ta, stream));
             }
@@ -2076,6 +2109,8 @@ struct Engine final : EngineBase {
         if (P.use_reservoir) ensure_planes(ck_n, (size_t)nck, rb);
         adj_ready = false;
         for (int64_t k = 0; k < nck; ++k) {
+            // the recompute starts from this copy, with the shape kept by then
+            if (adj_images() || !adj_recompute_tma || shape != kFusedShape + 8) need_images();
             plane_copy(*ck_psi[k], psi[0]);
             if (P.use_reservoir) plane_copy(*ck_n[k], nres[0]);
             const int64_t len = std::min(every, iterations - k * every);
@@ -2214,7 +2249,6 @@ struct Engine final : EngineBase {
         F.n1 = on ? rplane(*on) : nullptr;
         F.pump = P.n_pump_groups ? rplane(pump[0]) : nullptr;
         F.pot = P.n_potential_groups ? rplane(pot[0]) : nullptr;
-        F.st_images = !(adj_fused && MarchLauncher<T>::fits(plane) && AdjMarch<T>::wraps(N_c));
         for (int s = 0; s < 3; ++s) {
             F.st_psi[s] = cplane(*sp[s]);
             F.st_n[s] = sn[s] ? rplane(*sn[s]) : nullptr;

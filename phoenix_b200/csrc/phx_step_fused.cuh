@@ -50,7 +50,6 @@ struct FusedParams {
     T dt;
     cx<T>* st_psi[3];  // STORE: the stage values Y2..Y4 (with images), for the adjoint
     T* st_n[3];
-    int st_images;     // rk4_march_kernel: the stage values need their images (the others always write them)
 };
 
 constexpr int kImg = kImgDepth;

@@ -15,6 +15,7 @@
 //
 // The strip loses one column a side and stage, so 56 of its columns are stored;
 // a segment of L rows evaluates L + 6, L + 4, L + 2 and L rows.
+// (FP32 150, FP64 250 registers; four points per lane lost to the longer code.)
 //
 // Why: the tile kernels spend their time on stage barriers, on the stencil's
 // shared-memory traffic (70 % of that pipe) and on idle lanes in the
@@ -107,10 +108,14 @@ __device__ __forceinline__ void ring_two(const unsigned char* p, double* v) {
 // POT: the potential's terms are evaluated (an absent plane counts as zero).
 // UNIT: every temporal coefficient is exactly 1 (constant envelopes); the
 // products with it, which change nothing, are left out.  STORE: also write
-// the stage values Y2..Y4 of the stored points (with periodic images where
-// P.st_images), which the adjoint's backward sweep reads.  Plane indices are 32-bit (the host
-// takes this kernel for planes of fewer than 2^31 points only).
-template <typename T, bool RES, bool POT, bool UNIT, bool FMA, bool STORE>
+// the stage values Y2..Y4 of the stored points, which the adjoint's backward
+// sweep reads.  IMG: read the periodic images in the planes' rings and write
+// them for what is stored.  Without it (an even number of columns, or walls in
+// x) rows and column pairs wrap as they are copied, no image is read or
+// written, and a step has no branch left (FP32, us per iteration at 1024^2 /
+// 4096^2: 18.6 / 216 with, 16.2 / 184 without).  Plane indices are 32-bit (the
+// host takes this kernel for planes of fewer than 2^31 points only).
+template <typename T, bool RES, bool POT, bool UNIT, bool FMA, bool STORE, bool IMG>
 __device__ __forceinline__ void march_segment(const FusedParams<T>& P, int strip, int R0, int R1, unsigned char* ring) {
     using Lay = MarchLayout<T>;
     using C = cx<T>;
@@ -132,11 +137,14 @@ __device__ __forceinline__ void march_segment(const FusedParams<T>& P, int strip
     }
 
     // rows are counted from k = 0 at R0 - 4: step k evaluates stage s (0-based)
-    // on row k - s.  Lanes past the ring read its last columns: columns beyond
-    // N_c + 3 go wrong, which nothing stored depends on
-    const int last_k = R1 - R0 + 7;  // row R1 + 3, the last one that is read
-    int next_k = 0;                  // the next row to copy, and its place in the planes
-    int next_g = (R0 - 4) * pitch + min(c, (P.N_c + 8 - CPT) & ~(CPT - 1));
+    // on row k - s.  Copies run ahead to row R1 + 6, within the planes' rings of
+    // 8.  Lanes past the ring read its last columns: columns beyond N_c + 3 go
+    // wrong, which nothing stored depends on
+    const int last_k = R1 - R0 + 7;
+    const bool wrap_x = !IMG && P.img_x, wrap_y = !IMG && P.img_y;
+    int next_k = 0, next_r = R0 - 4;  // the next row to copy
+    if (wrap_y && next_r < 0) next_r += P.N_r;
+    int next_g = next_r * pitch + (wrap_x ? (c % P.N_c + P.N_c) % P.N_c : min(c, (P.N_c + 8 - CPT) & ~(CPT - 1)));
     const unsigned s_mine = (unsigned)__cvta_generic_to_shared(mine);
     auto issue = [&]() __attribute__((always_inline)) {
         const unsigned d = s_mine + (unsigned)(next_k & (kMarchRing - 1)) * Lay::row_bytes;
@@ -151,9 +159,10 @@ __device__ __forceinline__ void march_segment(const FusedParams<T>& P, int strip
             if (has_pot) cp_async<Lay::RB>(d + Lay::pot_off, P.pot + next_g);
         }
         cp_async_commit();
-        // past the last row the same one again: nothing reads it
-        next_g += next_k < last_k ? pitch : 0;
         ++next_k;
+        ++next_r;
+        next_g += pitch;
+        if (wrap_y && next_r == P.N_r) next_r = 0, next_g -= P.N_r * pitch;
     };
 #pragma unroll
     for (int k = 0; k < 5; ++k) issue();
@@ -173,6 +182,7 @@ __device__ __forceinline__ void march_segment(const FusedParams<T>& P, int strip
     auto put = [&](C* out, T* out_n, int row, const C* v, const T* nv) __attribute__((always_inline)) {
         const int g = row * pitch + c;
         if (store_lane) put_at(out, out_n, g, v, nv);
+        if constexpr (!IMG) return;
         if (edge_strip || (P.img_y && (row < kImg || row >= P.N_r - kImg))) {
             const int dy = !P.img_y ? 0 : (row < kImg ? P.N_r : (row >= P.N_r - kImg ? -P.N_r : 0));
             if (store_lane && dy) put_at(out, out_n, g + dy * pitch, v, nv);
@@ -258,8 +268,11 @@ __device__ __forceinline__ void march_segment(const FusedParams<T>& P, int strip
         }
         const int row = R0 - 4 + k - s;
         if constexpr (STORE && s < 3) {
-            if (store_lane && row >= R0 && row < R1) put_at(P.st_psi[own], P.st_n[own], row * pitch + c, o, on);
-            if (P.st_images && row >= R0 && row < R1) put(P.st_psi[own], P.st_n[own], row, o, on);
+            if constexpr (IMG) {
+                if (row >= R0 && row < R1) put(P.st_psi[own], P.st_n[own], row, o, on);
+            } else {
+                if (store_lane && row >= R0 && row < R1) put_at(P.st_psi[own], P.st_n[own], row * pitch + c, o, on);
+            }
         }
         if constexpr (s == 3) put(P.psi1, P.n1, row, o, on);
     };
@@ -293,7 +306,7 @@ __device__ __forceinline__ void march_segment(const FusedParams<T>& P, int strip
     for (; k < 7; ++k) step(std::integral_constant<int, 3>{}, k);
     // two steps a round: fewer register moves between the windows' rows, and a
     // loop that still comes from the instruction cache (FP32, us per iteration
-    // at 1024^2 / 4096^2: one step 19.2 / 224, two 18.9 / 218, three 18.7 / 222)
+    // at 1024^2 / 4096^2: one step 16.8 / 196, two 16.2 / 184)
 #pragma unroll 1
     while (k < last_k) {
         step(std::integral_constant<int, 4>{}, k);
@@ -306,7 +319,7 @@ __device__ __forceinline__ void march_segment(const FusedParams<T>& P, int strip
     cp_async_wait<0>();
 }
 
-template <typename T, bool RES, bool POT, bool UNIT, bool FMA, bool STORE, int MINB>
+template <typename T, bool RES, bool POT, bool UNIT, bool FMA, bool STORE, bool IMG, int MINB>
 __global__ void __launch_bounds__(32 * kMarchWarps, MINB) rk4_march_kernel(const __grid_constant__ MarchParams<T> Q) {
     extern __shared__ __align__(16) unsigned char march_smem[];
     const int warp = threadIdx.x >> 5, item = blockIdx.x * kMarchWarps + warp;
@@ -317,7 +330,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB) rk4_march_kernel(const
     // free slots leave the next grid unevenly spread over the SMs (25.4 against
     // 18.6 us at 1024^2 FP32, two CTAs per SM).
     pdl_wait();
-    march_segment<T, RES, POT, UNIT, FMA, STORE>(Q.f, item % Q.strips, R0, min(R0 + Q.seg_rows, Q.f.N_r),
+    march_segment<T, RES, POT, UNIT, FMA, STORE, IMG>(Q.f, item % Q.strips, R0, min(R0 + Q.seg_rows, Q.f.N_r),
                                                  march_smem + warp * MarchLayout<T>::warp_bytes);
 }
 
@@ -335,14 +348,14 @@ struct MarchBatchParams {
     int n_items, dir;
 };
 
-template <typename T, bool RES, bool POT, bool FMA, int MINB>
+template <typename T, bool RES, bool POT, bool FMA, bool IMG, int MINB>
 __global__ void __launch_bounds__(32 * kMarchWarps, MINB) rk4_march_batch_kernel(const __grid_constant__ MarchBatchParams<T> Q) {
     extern __shared__ __align__(16) unsigned char march_smem[];
     const int warp = threadIdx.x >> 5, item = blockIdx.x * kMarchWarps + warp;
     if (item >= Q.n_items) return;
     const MarchItem it = Q.items[item];
     const FusedParams<T> P = Q.f[2 * it.inst + Q.dir];
-    march_segment<T, RES, POT, true, FMA, false>(P, it.strip, it.r0, it.r1, march_smem + warp * MarchLayout<T>::warp_bytes);
+    march_segment<T, RES, POT, true, FMA, false, IMG>(P, it.strip, it.r0, it.r1, march_smem + warp * MarchLayout<T>::warp_bytes);
 }
 
 }  // namespace phx

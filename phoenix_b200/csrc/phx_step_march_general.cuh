@@ -73,7 +73,7 @@ struct MarchSrc {
     __device__ __forceinline__ cx<T> pulse(int g) const { return ps[g][0][j]; }
 };
 
-template <typename T, int COMPS, bool RES, int NP, int NV, int NQ, bool NOISE, bool REALV, int MINB>
+template <typename T, int COMPS, bool RES, int NP, int NV, int NQ, bool NOISE, bool REALV, bool IMG, int MINB>
 __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
     rk4_march_general_kernel(const __grid_constant__ MarchGeneralParams<T, COMPS> F) {
     using Lay = MarchGeneralLayout<T, COMPS, RES, NP, NV, NQ, NOISE>;
@@ -92,8 +92,10 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
 
     // rows are counted from k = 0 at R0 - 4: step k evaluates stage s (0-based) on row k - s
     const int last_k = R1 - R0 + 7;
-    int next_k = 0;
-    int next_g = (R0 - 4) * pitch + min(c, (N_c + 8 - CPT) & ~(CPT - 1));
+    const bool wrap_x = !IMG && P0.img_x, wrap_y = !IMG && P0.img_y;  // march_segment's IMG
+    int next_k = 0, next_r = R0 - 4;
+    if (wrap_y && next_r < 0) next_r += N_r;
+    int next_g = next_r * pitch + (wrap_x ? (c % N_c + N_c) % N_c : min(c, (N_c + 8 - CPT) & ~(CPT - 1)));
     auto copy_cx = [&](unsigned d, const C* p) __attribute__((always_inline)) {
 #pragma unroll
         for (int i = 0; i < PB / 16; ++i) cp_async<16>(d + i * 512, reinterpret_cast<const unsigned char*>(p + next_g) + i * 16);
@@ -114,8 +116,10 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
             for (int g = 0; g < NQ; ++g) copy_cx(d + Lay::pulse_off(g, q), (q ? F.st[0].pulse : P0.pulse) + g * plane);
         }
         cp_async_commit();
-        next_g += next_k < last_k ? pitch : 0;  // past the last row the same one again: nothing reads it
         ++next_k;
+        ++next_r;
+        next_g += pitch;
+        if (wrap_y && next_r == N_r) next_r = 0, next_g -= N_r * pitch;
     };
     pdl_wait();  // the previous iteration's kernel has completed
 #pragma unroll
@@ -137,7 +141,9 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
                 if constexpr (RES) out_n[gi] = nv[0];
             }
         };
-        if (store_lane) put_at(g);
+        if (store_lane && row >= R0) put_at(g);
+        if constexpr (!IMG) return;
+        if (row < R0) return;
         if (edge_strip || (P0.img_y && (row < kImgDepth || row >= N_r - kImgDepth))) {
             const int dy = !P0.img_y ? 0 : (row < kImgDepth ? N_r : (row >= N_r - kImgDepth ? -N_r : 0));
             if (store_lane && dy) put_at(g + dy * pitch);
@@ -289,11 +295,9 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
                 dn[q][j] = o[q][j];
             }
         if constexpr (s == 3) {
-            // a segment's first steps make no row of its own yet
-            if (row >= R0) {
+            // a segment's first steps make no row of its own yet (put)
 #pragma unroll
-                for (int q = 0; q < COMPS; ++q) put(q, row, o[q], on[q]);
-            }
+            for (int q = 0; q < COMPS; ++q) put(q, row, o[q], on[q]);
         }
     };
     // Every step runs all four stages: in a segment's first six steps the later
