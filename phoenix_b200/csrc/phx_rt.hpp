@@ -58,8 +58,9 @@ struct DevBuf {
         owned = false;
     }
     void alloc(size_t n, cudaStream_t s) {
-        if (p) cudaFree(p);
+        if (p && owned) cudaFree(p);
         p = nullptr;
+        owned = true;
         bytes = n;
         if (n == 0) return;
         cudaError_t e = cudaMalloc(&p, n);

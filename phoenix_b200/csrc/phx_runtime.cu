@@ -157,7 +157,9 @@ struct Engine final : EngineBase {
     int H = 4;  // halo width the reference uses: k_max of the iterator
     Tableau tab;  // the fixed-step tableau of the other iterators
 
-    // state and work planes (each allocation holds 1 or more planes)
+    // state and work planes (1 or more planes each), parts of `slab`
+    DevBuf slab;
+    static constexpr size_t kSlabBytes = (size_t)32 << 20;
     DevBuf psi[2], nres[2];            // state per component
     DevBuf sbuf_psi[2][2], sbuf_n[2][2];  // [component][ping-pong] stage values
     DevBuf acc_psi[2], acc_n[2];       // RK4 accumulators
@@ -211,28 +213,36 @@ struct Engine final : EngineBase {
         pitch = ((N_c + 2LL * G) + 31) / 32 * 32;
         rows = N_r + 2LL * G;
         plane = pitch * rows;
+        adj_fused = adj_fused && MarchLauncher<T>::fits(plane);
         d = derive<T>(P);
         PHX_CUDA(cudaSetDevice(P.device));
         PHX_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        // Every buffer of known size, out of one allocation where they are large: a
+        // cudaMalloc of its own for each took most of such a handle's set-up time.
+        // Small ones come cheaper one by one, out of the driver's pool.
+        std::vector<std::pair<DevBuf*, size_t>> parts;
+        auto want = [&](DevBuf& b, size_t n) { parts.push_back({&b, n}); };
         const size_t cb = sizeof(C) * plane, rb = sizeof(T) * plane;
         for (int q = 0; q < comps; ++q) {
-            psi[q].alloc(cb, stream);
-            nres[q].alloc(rb, stream);
+            want(psi[q], cb);
+            want(nres[q], rb);
             for (int b = 0; b < 2; ++b) {
-                sbuf_psi[q][b].alloc(cb, stream);
-                sbuf_n[q][b].alloc(rb, stream);
+                want(sbuf_psi[q][b], cb);
+                want(sbuf_n[q][b], rb);
             }
             if (P.iterator == PHX_ITER_RK4 && !imag_time()) {
-                acc_psi[q].alloc(cb, stream);
-                acc_n[q].alloc(rb, stream);
+                want(acc_psi[q], cb);
+                want(acc_n[q], rb);
+                want(psi_alt[q], cb);
+                want(n_alt[q], rb);
             } else {
                 const int kp = std::max({7, tab.H, tab.nb, tab.E});
-                k_psi[q].alloc(cb * kp, stream);
-                k_n[q].alloc(rb * kp, stream);
+                want(k_psi[q], cb * kp);
+                want(k_n[q], rb * kp);
             }
-            pump[q].alloc(rb * std::max(1, P.n_pump_groups), stream);
-            pot[q].alloc(rb * std::max(1, P.n_potential_groups), stream);
-            pulse[q].alloc(cb * std::max(1, P.n_pulse_groups), stream);
+            want(pump[q], rb * std::max(1, P.n_pump_groups));
+            want(pot[q], rb * std::max(1, P.n_potential_groups));
+            want(pulse[q], cb * std::max(1, P.n_pulse_groups));
         }
         long long min_rpb = rows_per_block(0);
         for (int sh = 1; sh < kShapes; ++sh) min_rpb = std::min(min_rpb, rows_per_block(sh));
@@ -248,14 +258,25 @@ struct Engine final : EngineBase {
             auto it = tune_cache().find(tune_key());
             if (it != tune_cache().end()) shape = it->second;
         }
-        partials.alloc(sizeof(double) * 2 * std::max<long long>(max_blocks, 1024), stream);
-        result.alloc(sizeof(double) * 4, stream);
+        want(partials, sizeof(double) * 2 * std::max<long long>(max_blocks, 1024));
+        want(result, sizeof(double) * 4);
+        want(imag_f, sizeof(double) * 2);
+        // zeroed with the handle: check_err_flag reads it past the stream's queue
+        // and must never see what the memory held before
+        if (fused_eligible_static()) want(err_flag, sizeof(int));
+        size_t total = 0;
+        for (auto& part : parts) total += (part.second + 511) / 512 * 512;
+        if (total >= kSlabBytes) {
+            slab.alloc(total, stream);
+            char* at = static_cast<char*>(slab.p);
+            for (auto& part : parts) {
+                part.first->view(at, part.second);
+                at += (part.second + 511) / 512 * 512;
+            }
+        } else {
+            for (auto& part : parts) part.first->alloc(part.second, stream);
+        }
         host_result.alloc(sizeof(double) * 4);
-        imag_f.alloc(sizeof(double) * 2, stream);
-        // set up here, not at the first launch that needs it: check_err_flag
-        // reads it past the stream's queue, and must never see what the
-        // memory held before
-        if (fused_eligible_static()) err_flag.alloc(sizeof(int), stream);
         t = (T)P.t0;
         dt = (T)P.dt;
         fft_cached_t = (T)0.0;
@@ -866,7 +887,7 @@ struct Engine final : EngineBase {
         images_ok = true;
     }
     // the adjoint's planes need images where its sweep does not wrap
-    bool adj_images() const { return !(adj_fused && MarchLauncher<T>::fits(plane) && AdjMarch<T>::wraps(N_c)); }
+    bool adj_images() const { return !(adj_fused && AdjMarch<T>::wraps(N_c)); }
     void go_march(const FusedParams<T>& F, bool res, bool fma, bool store = false) {
         const bool img = march_needs_images(N_c, P.periodic_x) || (store && adj_images());
         if (!store) {
@@ -951,7 +972,6 @@ struct Engine final : EngineBase {
                 F.pot_c[s] = c.real();
             }
         }
-        ensure_alt();
         fused_constants<T>(F, P, d, dt, pitch);
         F.psi0 = cplane(psi[0]);
         F.n0 = rplane(nres[0]);
@@ -988,13 +1008,6 @@ struct Engine final : EngineBase {
     }
     // The one-kernel iterations write the other of two state planes, and of its
     // ring only the periodic images: the zeros along zero axes stay.
-    void ensure_alt() {
-        for (int q = 0; q < comps; ++q)
-            if (!psi_alt[q].p) {
-                psi_alt[q].alloc(sizeof(C) * plane, stream);
-                n_alt[q].alloc(sizeof(T) * plane, stream);
-            }
-    }
     void swap_alt() {
         for (int q = 0; q < comps; ++q) {
             std::swap(psi[q].p, psi_alt[q].p);
@@ -1047,7 +1060,6 @@ struct Engine final : EngineBase {
         const T cw[4] = {(T)0.0, (T)0.5, (T)0.5, (T)1.0};
         const T aw[3] = {(T)0.5, (T)0.5, (T)1.0};
         const T bw[4] = {(T)(1.0 / 6.0), (T)(1.0 / 3.0), (T)(1.0 / 3.0), (T)(1.0 / 6.0)};
-        ensure_alt();
         TetmFusedParams<T> F;
         std::memset(&F, 0, sizeof(F));
         for (int s = 1; s <= 4; ++s) {
@@ -1115,7 +1127,6 @@ struct Engine final : EngineBase {
         const T cw[4] = {(T)0.0, (T)0.5, (T)0.5, (T)1.0};
         const T aw[3] = {(T)0.5, (T)0.5, (T)1.0};
         const T bw[4] = {(T)(1.0 / 6.0), (T)(1.0 / 3.0), (T)(1.0 / 3.0), (T)(1.0 / 6.0)};
-        ensure_alt();
         TetmParams<T> st[4];
         std::memset(st, 0, sizeof(st));
         for (int s = 1; s <= 4; ++s) {
@@ -2063,8 +2074,8 @@ struct Engine final : EngineBase {
     int64_t adj_T = 0, adj_every = 0;
     T adj_dt = 0;
     bool adj_ready = false;
-    // one fused launch per iteration (adj_fused_kernel); PHX_ADJOINT_STAGES=1
-    // selects the four-launch path (adj_stage_kernel)
+    // one launch per iteration (adj_march_kernel); PHX_ADJOINT_STAGES=1, or planes
+    // beyond 32-bit indices, select the four-launch path (adj_stage_kernel)
     bool adj_fused = !(std::getenv("PHX_ADJOINT_STAGES") && std::atoi(std::getenv("PHX_ADJOINT_STAGES")) == 1);
     bool adj_recompute_tma =
         !(std::getenv("PHX_ADJOINT_RECOMPUTE") && std::string(std::getenv("PHX_ADJOINT_RECOMPUTE")) == "fused");
@@ -2445,21 +2456,7 @@ struct Engine final : EngineBase {
                     cudaEvent_t a = nullptr;
                     prof_begin(a);
                     if (!sm_count) PHX_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, P.device));
-                    auto go_adj = [&](auto tw, auto th, auto nt, auto minb) {
-                        constexpr int TW = decltype(tw)::value, TH = decltype(th)::value, NT = decltype(nt)::value;
-                        constexpr int MINB = decltype(minb)::value;
-                        dim3 grid((unsigned)((N_c + TW - 1) / TW), (unsigned)((N_r + TH - 1) / TH));
-                        adj_fused_kernel<T, TW, TH, NT, MINB><<<grid, NT, 0, stream>>>(Q);
-                    };
-                    using std::integral_constant;
-                    if (MarchLauncher<T>::fits(plane))
-                        adj_march.launch(Q, sm_count, stream, pdl_on());
-                    else if constexpr (sizeof(T) == 4)  // 64 x 16 tiles, 16 warps, two CTAs per SM
-                        go_adj(integral_constant<int, 64>{}, integral_constant<int, 16>{}, integral_constant<int, 512>{},
-                               integral_constant<int, 2>{});
-                    else
-                        go_adj(integral_constant<int, 32>{}, integral_constant<int, 16>{}, integral_constant<int, 256>{},
-                               integral_constant<int, 1>{});
+                    adj_march.launch(Q, sm_count, stream, pdl_on());
                     prof_end(PHX_KERNEL_OTHER, a, (double)N_r * N_c * (5.0 * sizeof(C) + 7.0 * sizeof(T)));
                     ++launches;
                     PHX_CUDA(cudaGetLastError());
