@@ -159,7 +159,6 @@ struct Engine final : EngineBase {
 
     // state and work planes (1 or more planes each), parts of `slab`
     DevBuf slab;
-    static constexpr size_t kSlabBytes = (size_t)32 << 20;
     DevBuf psi[2], nres[2];            // state per component
     DevBuf sbuf_psi[2][2], sbuf_n[2][2];  // [component][ping-pong] stage values
     DevBuf acc_psi[2], acc_n[2];       // RK4 accumulators
@@ -217,9 +216,8 @@ struct Engine final : EngineBase {
         d = derive<T>(P);
         PHX_CUDA(cudaSetDevice(P.device));
         PHX_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-        // Every buffer of known size, out of one allocation where they are large: a
-        // cudaMalloc of its own for each took most of such a handle's set-up time.
-        // Small ones come cheaper one by one, out of the driver's pool.
+        // Every buffer of known size, out of one allocation: a cudaMalloc of its own
+        // for each took most of the handle's set-up time.
         std::vector<std::pair<DevBuf*, size_t>> parts;
         auto want = [&](DevBuf& b, size_t n) { parts.push_back({&b, n}); };
         const size_t cb = sizeof(C) * plane, rb = sizeof(T) * plane;
@@ -266,15 +264,11 @@ struct Engine final : EngineBase {
         if (fused_eligible_static()) want(err_flag, sizeof(int));
         size_t total = 0;
         for (auto& part : parts) total += (part.second + 511) / 512 * 512;
-        if (total >= kSlabBytes) {
-            slab.alloc(total, stream);
-            char* at = static_cast<char*>(slab.p);
-            for (auto& part : parts) {
-                part.first->view(at, part.second);
-                at += (part.second + 511) / 512 * 512;
-            }
-        } else {
-            for (auto& part : parts) part.first->alloc(part.second, stream);
+        slab.alloc(total, stream);
+        char* at = static_cast<char*>(slab.p);
+        for (auto& part : parts) {
+            part.first->view(at, part.second);
+            at += (part.second + 511) / 512 * 512;
         }
         host_result.alloc(sizeof(double) * 4);
         t = (T)P.t0;

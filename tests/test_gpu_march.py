@@ -116,3 +116,34 @@ def test_general_and_spinor_iterations(require_gpu, monkeypatch, tetm, dtype, pu
         got = general(n_c, n_r, dtype, px, py, monkeypatch, False, tetm, pumps, pot, pulse, dw)
         for x, y in zip(got, want):
             np.testing.assert_array_equal(x, y, err_msg=f"{n_c} x {n_r}")
+
+
+# the adjoint's vector-Jacobian kernel: strips of 56 columns, wrapping (even
+# widths) and with periodic images (odd ones), against the four-launch form.
+# FP64: the two differ in the order of a few sums, 1e-12 as in the adjoint's own
+# tests; FP32: 5 iterations of some 100 rounded operations a stage, 2e-5.
+@pytest.mark.parametrize("n_c,n_r,dtype,tol", [(8, 8, "f64", 1e-12), (57, 33, "f64", 1e-12), (56, 41, "f64", 1e-12),
+                                               (113, 70, "f64", 1e-12), (114, 75, "f32", 2e-5), (58, 9, "f32", 2e-5)])
+def test_adjoint_sweep(require_gpu, monkeypatch, n_c, n_r, dtype, tol):
+    import torch
+
+    rng = np.random.default_rng([n_c, n_r, 5])
+    ct, rt = (torch.complex64, torch.float32) if dtype == "f32" else (torch.complex128, torch.float64)
+    z = lambda: torch.tensor(rng.standard_normal((n_r, n_c)) + 1j * rng.standard_normal((n_r, n_c))).to(ct).cuda()  # noqa: E731
+    r = lambda: torch.tensor(rng.random((n_r, n_c))).to(rt).cuda()  # noqa: E731
+    psi0, n0, pump, pot, d_psi, d_n = z(), r(), r(), r(), z(), r()
+    got = {}
+    for stages in ("1", "0"):
+        monkeypatch.setenv("PHX_ADJOINT_STAGES", stages)
+        sp = pb.SystemParameters(N_c=n_c, N_r=n_r, L_x=0.3 * n_c, L_y=0.3 * n_r, **B.PHYS, periodic_boundary_x=True,
+                                 periodic_boundary_y=True, dtype=dtype, dt=0.01, t_max=1e12, fft_every=1e12,
+                                 pump_temporal=[pb.Temporal()], potential_temporal=[pb.Temporal()])
+        with pb.Solver(sp) as s:
+            s.set_field_tensor("pump_plus", pump)
+            s.set_field_tensor("potential_plus", pot)
+            s.set_field_tensor("psi_plus", psi0)
+            s.set_field_tensor("n_plus", n0)
+            s.adjoint_forward(5, 2)
+            got[stages] = s.adjoint_backward(d_psi, d_n, want_potential=True)
+    for a, b in zip(got["0"], got["1"]):
+        assert float((a - b).norm() / b.norm()) <= tol
