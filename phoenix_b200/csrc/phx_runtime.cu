@@ -166,7 +166,7 @@ struct Engine final : EngineBase {
     DevBuf pump[2], pot[2], pulse[2];  // input planes (groups)
     DevBuf mask[2];                    // fft-shifted mask, contiguous N_r*N_c
     DevBuf fft_x;                      // contiguous scratch for the filter
-    DevBuf psi_alt[2], n_alt[2];       // second state planes of the one-kernel RK4 iterations
+    DevBuf psi_alt[2], n_alt[2];       // second state planes of the tuned one-kernel RK4 iterations (alt_psi)
     DevBuf err_flag;                   // set by kernels whose bounded waits gave up
     DevBuf partials, result;
     PinnedBuf host_result;
@@ -221,30 +221,6 @@ struct Engine final : EngineBase {
         std::vector<std::pair<DevBuf*, size_t>> parts;
         auto want = [&](DevBuf& b, size_t n) { parts.push_back({&b, n}); };
         const size_t cb = sizeof(C) * plane, rb = sizeof(T) * plane;
-        for (int q = 0; q < comps; ++q) {
-            want(psi[q], cb);
-            want(nres[q], rb);
-            for (int b = 0; b < 2; ++b) {
-                want(sbuf_psi[q][b], cb);
-                want(sbuf_n[q][b], rb);
-            }
-            if (P.iterator == PHX_ITER_RK4 && !imag_time()) {
-                want(acc_psi[q], cb);
-                want(acc_n[q], rb);
-                want(psi_alt[q], cb);
-                want(n_alt[q], rb);
-            } else {
-                const int kp = std::max({7, tab.H, tab.nb, tab.E});
-                want(k_psi[q], cb * kp);
-                want(k_n[q], rb * kp);
-            }
-            want(pump[q], rb * std::max(1, P.n_pump_groups));
-            want(pot[q], rb * std::max(1, P.n_potential_groups));
-            want(pulse[q], cb * std::max(1, P.n_pulse_groups));
-        }
-        long long min_rpb = rows_per_block(0);
-        for (int sh = 1; sh < kShapes; ++sh) min_rpb = std::min(min_rpb, rows_per_block(sh));
-        const long long max_blocks = grid_x(-(long long)G, N_c + G) * ((N_r + 2LL * G + min_rpb - 1) / min_rpb) + kRingBlocks;
         if (const char* e = std::getenv("PHX_STAGE_SHAPE")) {
             const int v = std::atoi(e);
             if (v >= 0 && v < kShapes) shape = v;
@@ -256,6 +232,33 @@ struct Engine final : EngineBase {
             auto it = tune_cache().find(tune_key());
             if (it != tune_cache().end()) shape = it->second;
         }
+        for (int q = 0; q < comps; ++q) {
+            want(psi[q], cb);
+            want(nres[q], rb);
+            for (int b = 0; b < 2; ++b) {
+                want(sbuf_psi[q][b], cb);
+                want(sbuf_n[q][b], rb);
+            }
+            if (P.iterator == PHX_ITER_RK4 && !imag_time()) {
+                want(acc_psi[q], cb);
+                want(acc_n[q], rb);
+                // see alt_psi: a plane of its own only where stage kernels may step in
+                if (fused_eligible_static() && (shape < 0 || is_fused(shape))) {
+                    want(psi_alt[q], cb);
+                    want(n_alt[q], rb);
+                }
+            } else if (P.iterator != PHX_ITER_SSFM) {  // which keeps no k-stack
+                const int kp = std::max({7, tab.H, tab.nb, tab.E});
+                want(k_psi[q], cb * kp);
+                want(k_n[q], rb * kp);
+            }
+            want(pump[q], rb * std::max(1, P.n_pump_groups));
+            want(pot[q], rb * std::max(1, P.n_potential_groups));
+            want(pulse[q], cb * std::max(1, P.n_pulse_groups));
+        }
+        long long min_rpb = rows_per_block(0);
+        for (int sh = 1; sh < kShapes; ++sh) min_rpb = std::min(min_rpb, rows_per_block(sh));
+        const long long max_blocks = grid_x(-(long long)G, N_c + G) * ((N_r + 2LL * G + min_rpb - 1) / min_rpb) + kRingBlocks;
         want(partials, sizeof(double) * 2 * std::max<long long>(max_blocks, 1024));
         want(result, sizeof(double) * 4);
         want(imag_f, sizeof(double) * 2);
@@ -969,8 +972,8 @@ struct Engine final : EngineBase {
         fused_constants<T>(F, P, d, dt, pitch);
         F.psi0 = cplane(psi[0]);
         F.n0 = rplane(nres[0]);
-        F.psi1 = cplane(psi_alt[0]);
-        F.n1 = rplane(n_alt[0]);
+        F.psi1 = cplane(alt_psi(0));
+        F.n1 = rplane(alt_n(0));
         F.pump = P.n_pump_groups ? rplane(pump[0]) : nullptr;
         F.pot = P.n_potential_groups ? rplane(pot[0]) : nullptr;
         cudaEvent_t a = nullptr;
@@ -1001,11 +1004,17 @@ struct Engine final : EngineBase {
         return true;
     }
     // The one-kernel iterations write the other of two state planes, and of its
-    // ring only the periodic images: the zeros along zero axes stay.
+    // ring only the periodic images: the zeros along zero axes stay.  Iterations
+    // that the stage kernels never take over (TE/TM, noise, pulses, several
+    // groups) write the first stage plane, which they have no other use for; where
+    // complex envelopes can hand an iteration to the stage kernels, which leave
+    // stage values in their planes' rings, the second state has its own plane.
+    DevBuf& alt_psi(int q) { return psi_alt[q].p ? psi_alt[q] : sbuf_psi[q][0]; }
+    DevBuf& alt_n(int q) { return n_alt[q].p ? n_alt[q] : sbuf_n[q][0]; }
     void swap_alt() {
         for (int q = 0; q < comps; ++q) {
-            std::swap(psi[q].p, psi_alt[q].p);
-            std::swap(nres[q].p, n_alt[q].p);
+            std::swap(psi[q].p, alt_psi(q).p);
+            std::swap(nres[q].p, alt_n(q).p);
         }
     }
     // the marching-warps form of an iteration the kernels below also take
@@ -1019,8 +1028,8 @@ struct Engine final : EngineBase {
         for (int q = 0; q < comps; ++q) {
             p0[q] = cplane(psi[q]);
             n0[q] = rplane(nres[q]);
-            p1[q] = cplane(psi_alt[q]);
-            n1[q] = rplane(n_alt[q]);
+            p1[q] = cplane(alt_psi(q));
+            n1[q] = rplane(alt_n(q));
         }
         const bool img = march_needs_images(N_c, P.periodic_x);
         if (img) need_images();
@@ -1075,8 +1084,8 @@ struct Engine final : EngineBase {
         for (int q = 0; q < 2; ++q) {
             F.psi0[q] = cplane(psi[q]);
             F.n0[q] = rplane(nres[q]);
-            F.psi1[q] = cplane(psi_alt[q]);
-            F.n1[q] = rplane(n_alt[q]);
+            F.psi1[q] = cplane(alt_psi(q));
+            F.n1[q] = rplane(alt_n(q));
         }
         cudaEvent_t a = nullptr;
         prof_begin(a);
@@ -1143,8 +1152,8 @@ struct Engine final : EngineBase {
             for (int s = 0; s < 4; ++s) F.st[s] = st[s].p;
             F.psi0 = cplane(psi[0]);
             F.n0 = rplane(nres[0]);
-            F.psi1 = cplane(psi_alt[0]);
-            F.n1 = rplane(n_alt[0]);
+            F.psi1 = cplane(alt_psi(0));
+            F.n1 = rplane(alt_n(0));
             constexpr bool f32 = sizeof(T) == 4;
             if (P.use_reservoir)
                 go_general<true, 32, f32 ? 16 : 8, 512>(F);
