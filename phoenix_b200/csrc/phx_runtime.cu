@@ -211,6 +211,11 @@ struct Engine final : EngineBase {
         G = std::max(kRing, H + 1);
         pitch = ((N_c + 2LL * G) + 31) / 32 * 32;
         rows = N_r + 2LL * G;
+        if (P.iterator == PHX_ITER_SSFM) {  // no stencil, no ring: planes as the transforms want them
+            G = 0;
+            pitch = N_c;
+            rows = N_r;
+        }
         plane = pitch * rows;
         adj_fused = adj_fused && MarchLauncher<T>::fits(plane);
         d = derive<T>(P);
@@ -1709,43 +1714,31 @@ struct Engine final : EngineBase {
 
     // ------------------------------------------------------------ SSFM
     // SSFM::step (split_step_fourier_method.cu:24-72): four unnormalised
-    // transforms per iteration on contiguous copies of psi, with the
-    // reference's (N_c, N_r) plan; kernels in phx_ssfm.cuh.
-    DevBuf ssfm_w[2], ssfm_f[2];  // contiguous copies, other than square grids only
-    DevBuf ssfm_table;            // the linear half step's factors for ssfm_table_dt
+    // transforms per iteration in place on the psi planes, with the reference's
+    // (N_c, N_r) plan; kernels in phx_ssfm.cuh.
+    DevBuf ssfm_table;  // the linear half step's factors for ssfm_table_dt
     T ssfm_table_dt = 0;
     cufftHandle ssfm_plan = 0;
     bool have_ssfm_plan = false;
-    void ssfm_fft(C* in, C* out, int dir) {
+    void ssfm_fft(C* psi_q, int dir) {
         if constexpr (sizeof(T) == 4) {
-            PHX_CUFFT(cufftExecC2C(ssfm_plan, reinterpret_cast<cufftComplex*>(in), reinterpret_cast<cufftComplex*>(out), dir));
+            auto* p = reinterpret_cast<cufftComplex*>(psi_q);
+            PHX_CUFFT(cufftExecC2C(ssfm_plan, p, p, dir));
         } else {
-            PHX_CUFFT(cufftExecZ2Z(ssfm_plan, reinterpret_cast<cufftDoubleComplex*>(in), reinterpret_cast<cufftDoubleComplex*>(out),
-                                   dir));
+            auto* p = reinterpret_cast<cufftDoubleComplex*>(psi_q);
+            PHX_CUFFT(cufftExecZ2Z(ssfm_plan, p, p, dir));
         }
     }
     void step_ssfm() {
         const long long N = (long long)N_r * N_c;
-        const bool square = N_r == N_c && plane < (1LL << 31);
         if (!have_ssfm_plan) {
-            if (square) {
-                int n[2] = {N_r, N_c}, embed[2] = {(int)rows, (int)pitch};
-                PHX_CUFFT(cufftPlanMany(&ssfm_plan, 2, n, embed, 1, (int)plane, embed, 1, (int)plane,
-                                        sizeof(T) == 4 ? CUFFT_C2C : CUFFT_Z2Z, 1));
-            } else {
-                for (int q = 0; q < comps; ++q) {
-                    ssfm_w[q].alloc(sizeof(C) * N, stream);
-                    ssfm_f[q].alloc(sizeof(C) * N, stream);
-                }
-                PHX_CUFFT(cufftPlan2d(&ssfm_plan, N_c, N_r, sizeof(T) == 4 ? CUFFT_C2C : CUFFT_Z2Z));
-            }
+            PHX_CUFFT(cufftPlan2d(&ssfm_plan, N_c, N_r, sizeof(T) == 4 ? CUFFT_C2C : CUFFT_Z2Z));
             PHX_CUFFT(cufftSetStream(ssfm_plan, stream));
             have_ssfm_plan = true;
         }
         SsfmParams<T> S;
         std::memset(&S, 0, sizeof(S));
-        S.N_r = N_r, S.N_c = N_c, S.pitch = pitch, S.tetm = P.tetm, S.res = P.use_reservoir;
-        S.wp = square ? pitch : N_c;
+        S.N_r = N_r, S.N_c = N_c, S.tetm = P.tetm, S.res = P.use_reservoir;
         S.hbs = (T)P.h_bar_s, S.meff = (T)P.m_eff, S.Lx = (T)P.L_x, S.Ly = (T)P.L_y, S.dt = dt, S.N2 = (T)(unsigned)N;
         S.g_c = (T)P.g_c, S.g_r = (T)P.g_r, S.R = (T)P.R, S.gamma_c = (T)P.gamma_c, S.gamma_r = (T)P.gamma_r;
         S.g_pm = (T)P.g_pm, S.ohb = d.ohb, S.dV = d.dV;
@@ -1765,10 +1758,7 @@ struct Engine final : EngineBase {
         S.noise_amp = B.noise_amp;
         S.periodic_x = P.periodic_x, S.periodic_y = P.periodic_y;
         const int blocks = (int)std::min<long long>((N + 255) / 256, 148 * 16);
-        C* w[2] = {reinterpret_cast<C*>(ssfm_w[0].p), comps > 1 ? reinterpret_cast<C*>(ssfm_w[1].p) : nullptr};
-        C* f[2] = {reinterpret_cast<C*>(ssfm_f[0].p), comps > 1 ? reinterpret_cast<C*>(ssfm_f[1].p) : nullptr};
-        if (square)
-            for (int q = 0; q < comps; ++q) w[q] = f[q] = cplane(psi[q]);
+        C* w[2] = {cplane(psi[0]), comps > 1 ? cplane(psi[1]) : nullptr};
         cudaEvent_t a = nullptr;
         prof_begin(a);
         if (!ssfm_table.p || ssfm_table_dt != dt) {
@@ -1780,28 +1770,23 @@ struct Engine final : EngineBase {
         const C* table = reinterpret_cast<const C*>(ssfm_table.p);
         // nothing left for the last kernel: the reservoir's update can go straight
         // into its plane (TE/TM runs never copy theirs back, noise scales with the old one)
-        const bool plain = square && !P.tetm && !S.n_pulse && !S.noise.on;
-        if (!square)
-            for (int q = 0; q < comps; ++q)
-                gather_interior_kernel<T><<<blocks, 256, 0, stream>>>(cplane(psi[q]), pitch, N_r, N_c, w[q]);
+        const bool plain = !P.tetm && !S.n_pulse && !S.noise.on;
+        T* rvp = rplane(nres[0]);
+        T* brvp = plain ? rvp : rplane(sbuf_n[0][0]);
+        T* brvm = comps > 1 ? rplane(sbuf_n[1][0]) : nullptr;
         for (int half = 0; half < 2; ++half) {
             for (int q = 0; q < comps; ++q) {
-                ssfm_fft(w[q], f[q], CUFFT_FORWARD);
-                ssfm_linear_kernel<T><<<blocks, 256, 0, stream>>>(S, table, f[q], w[q]);
-                ssfm_fft(w[q], f[q], CUFFT_INVERSE);
+                ssfm_fft(w[q], CUFFT_FORWARD);
+                ssfm_linear_kernel<T><<<blocks, 256, 0, stream>>>(S, table, w[q]);
+                ssfm_fft(w[q], CUFFT_INVERSE);
             }
             if (half == 1) break;
-            T* rvm = comps > 1 ? rplane(nres[1]) : nullptr;
-            T* brvm = comps > 1 ? rplane(sbuf_n[1][0]) : nullptr;
-            ssfm_nonlinear_kernel<T><<<blocks, 256, 0, stream>>>(S, f[0], f[1], rplane(nres[0]), rvm, w[0], w[1],
-                                                                 plain ? rplane(nres[0]) : rplane(sbuf_n[0][0]), brvm);
+            ssfm_nonlinear_kernel<T><<<blocks, 256, 0, stream>>>(S, w[0], w[1], rvp, comps > 1 ? rplane(nres[1]) : nullptr, brvp,
+                                                                 brvm);
         }
-        if (!plain)
-            ssfm_independent_kernel<T><<<blocks, 256, 0, stream>>>(S, f[0], f[1], rplane(nres[0]), rplane(sbuf_n[0][0]),
-                                                                   comps > 1 ? rplane(sbuf_n[1][0]) : nullptr, cplane(psi[0]),
-                                                                   comps > 1 ? cplane(psi[1]) : nullptr);
+        if (!plain) ssfm_independent_kernel<T><<<blocks, 256, 0, stream>>>(S, rvp, brvp, brvm, w[0], w[1]);
         prof_end(PHX_KERNEL_OTHER, a, (double)N * comps * 16 * sizeof(C));
-        launches += comps * (square ? 2 : 3) + (plain ? 1 : 2);
+        launches += comps * 2 + (plain ? 1 : 2);
         PHX_CUDA(cudaGetLastError());
     }
 
@@ -1827,7 +1812,7 @@ struct Engine final : EngineBase {
                 if (have_mask[q]) {
                     exec_fft(CUFFT_INVERSE);
                     scatter_interior_kernel<T><<<blocks, 256, 0, stream>>>(reinterpret_cast<C*>(fft_x.p), cplane(psi[q]), pitch, N_r,
-                                                                           N_c, P.periodic_x, P.periodic_y);
+                                                                           N_c, G && P.periodic_x, G && P.periodic_y);
                     ++launches;
                 }
                 prof_end(PHX_KERNEL_FILTER, a, (double)N * (6 * sizeof(C) + sizeof(T)));
@@ -1852,7 +1837,7 @@ struct Engine final : EngineBase {
             mask_kernel<T><<<blocks, 256, 0, stream>>>(reinterpret_cast<C*>(fft_x.p), reinterpret_cast<const T*>(mask[q].p), N);
             exec_fft(CUFFT_INVERSE);
             scatter_interior_kernel<T><<<blocks, 256, 0, stream>>>(reinterpret_cast<C*>(fft_x.p), cplane(psi[q]), pitch, N_r, N_c,
-                                                                   P.periodic_x, P.periodic_y);
+                                                                   G && P.periodic_x, G && P.periodic_y);
             prof_end(PHX_KERNEL_FILTER, a, (double)N * (6 * sizeof(C) + sizeof(T)));
             launches += 3;
             PHX_CUDA(cudaGetLastError());

@@ -1,10 +1,11 @@
 // Split-step Fourier iterator (the reference's "SSFM",
 // source/cuda_solver/solver/iterator/split_step_fourier_method.cu:24-72 with
-// the kernels of include/kernel/kernel_gp_compute.cuh:244-440).  Halo 0: four
-// unnormalised cuFFT transforms per iteration, with the (N_c, N_r) plan of
-// solver_fft.cu:102-118.  Square grids are transformed in place on the
-// halo-padded planes; other shapes as a contiguous N_r x N_c copy, which that
-// plan reads as N_c rows of N_r.  The reservoir stays in its padded plane.
+// the kernels of include/kernel/kernel_gp_compute.cuh:244-440).  Halo 0: the
+// planes of such a handle have no ring, and the four unnormalised cuFFT
+// transforms per iteration, with the (N_c, N_r) plan of solver_fft.cu:102-118,
+// run in place on them.  (On planes with a ring the transforms need a plan with
+// padded rows, which is up to 1.7 times as slow at some sizes: 24.8 us against
+// 14.6 at 500^2 FP32, 39 against 28 at 1280^2; copies in and out cost two passes.)
 //   linear half step   psi <- F^-1[ F[psi] / N2 exp(-i lin dt / 2) ],
 //                      lin = hbar / 2 / m (kx^2 + ky^2), k = 2 pi j / L with
 //                      the reference's literal pi = 3.1415926535
@@ -25,14 +26,12 @@ namespace phx {
 template <typename T>
 struct SsfmParams {
     int N_r, N_c;
-    long long pitch;     // of the padded planes
-    long long wp;        // row pitch of the transformed arrays: N_c, or pitch (in place on the padded planes)
     int tetm, res;
     T hbs, meff, Lx, Ly, dt, N2;
     T g_c, g_r, R, gamma_c, gamma_r, g_pm, ohb, dV;
     int n_pump, n_pot, n_pulse;
-    long long plane;     // group stride of the padded input planes
-    const T* pump[2];    // padded planes (interior origin), [component]
+    long long plane;     // group stride of the input planes: N_r * N_c
+    const T* pump[2];    // [component]
     const T* pot[2];
     const cx<T>* pulse[2];
     cx<T> amp_pump[kMaxGroups], amp_pot[kMaxGroups], amp_pulse[kMaxGroups];
@@ -70,15 +69,13 @@ __global__ void ssfm_table_kernel(const __grid_constant__ SsfmParams<T> S, cx<T>
         table[i] = cexp_dev(z);
     }
 }
-// gp_scalar_linear_fourier: out = in / N2 * table; rows of S.wp points
+// gp_scalar_linear_fourier: psi / N2 * table
 template <typename T>
-__global__ void ssfm_linear_kernel(const __grid_constant__ SsfmParams<T> S, const cx<T>* table, const cx<T>* in, cx<T>* out) {
+__global__ void ssfm_linear_kernel(const __grid_constant__ SsfmParams<T> S, const cx<T>* __restrict__ table, cx<T>* psi) {
     const long long N = (long long)S.N_r * S.N_c;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-        const unsigned r = (unsigned)i / (unsigned)S.N_c, c = (unsigned)i - r * (unsigned)S.N_c;  // at most 2^31 points
-        const long long w = r * S.wp + c;
-        const cx<T> a = in[w];
-        out[w] = cmul(mk(rdiv(a.re, S.N2), rdiv(a.im, S.N2)), table[i]);
+        const cx<T> a = psi[i];
+        psi[i] = cmul(mk(rdiv(a.re, S.N2), rdiv(a.im, S.N2)), table[i]);
     }
 }
 
@@ -114,66 +111,63 @@ __device__ __forceinline__ void ssfm_nonlinear_one(const SsfmParams<T>& S, int c
     out_rv = radd(in_rv, rmul(S.dt, r));
 }
 
-// gp_scalar_nonlinear: (fft, rv) -> (wf, buffer rv)
+// gp_scalar_nonlinear: (psi, rv) -> (psi, buffer rv)
 template <typename T>
-__global__ void ssfm_nonlinear_kernel(const __grid_constant__ SsfmParams<T> S, const cx<T>* fp, const cx<T>* fm,
-                                      const T* rvp, const T* rvm, cx<T>* wp, cx<T>* wm, T* brvp, T* brvm) {
+__global__ void ssfm_nonlinear_kernel(const __grid_constant__ SsfmParams<T> S, cx<T>* psip, cx<T>* psim, const T* rvp,
+                                      const T* rvm, T* brvp, T* brvm) {
     const long long N = (long long)S.N_r * S.N_c;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-        const unsigned r = (unsigned)i / (unsigned)S.N_c, c = (unsigned)i - r * (unsigned)S.N_c;  // at most 2^31 points
-        const long long pi = r * S.pitch + c, w = r * S.wp + c;
         if (!S.tetm) {
             cx<T> o;
             T on;
-            ssfm_nonlinear_one(S, 0, pi, fp[w], S.res ? rvp[pi] : (T)0, (T)0, o, on);
-            wp[w] = o;
-            if (S.res) brvp[pi] = on;
+            ssfm_nonlinear_one(S, 0, i, psip[i], S.res ? rvp[i] : (T)0, (T)0, o, on);
+            psip[i] = o;
+            if (S.res) brvp[i] = on;
         } else {
-            const cx<T> a = fp[w], b = fm[w];
+            const cx<T> a = psip[i], b = psim[i];
             cx<T> o;
             T on;
-            ssfm_nonlinear_one(S, 0, pi, a, rvp[pi], abs2(b), o, on);
-            wp[w] = o;
-            brvp[pi] = on;
-            ssfm_nonlinear_one(S, 1, pi, b, rvm[pi], abs2(a), o, on);
-            wm[w] = o;
-            brvm[pi] = on;
+            ssfm_nonlinear_one(S, 0, i, a, rvp[i], abs2(b), o, on);
+            psip[i] = o;
+            brvp[i] = on;
+            ssfm_nonlinear_one(S, 1, i, b, rvm[i], abs2(a), o, on);
+            psim[i] = o;
+            brvm[i] = on;
         }
     }
 }
 
-// gp_scalar_independent: psi = fft + pulse + dw into the padded state plane;
-// the scalar branch copies the buffer reservoir back, the TE/TM branch does not
+// gp_scalar_independent: psi = fft + pulse + dw; the scalar branch copies the
+// buffer reservoir back, the TE/TM branch does not
 template <typename T>
-__global__ void ssfm_independent_kernel(const __grid_constant__ SsfmParams<T> S, const cx<T>* fp,
-                                        const cx<T>* fm, T* rvp, const T* brvp, const T* brvm, cx<T>* psip, cx<T>* psim) {
+__global__ void ssfm_independent_kernel(const __grid_constant__ SsfmParams<T> S, T* rvp, const T* brvp, const T* brvm,
+                                        cx<T>* psip, cx<T>* psim) {
     const long long N = (long long)S.N_r * S.N_c;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-        const unsigned r = (unsigned)i / (unsigned)S.N_c, c = (unsigned)i - r * (unsigned)S.N_c;  // at most 2^31 points
-        const long long pi = r * S.pitch + c, w = r * S.wp + c;
         cx<T> ap = mk((T)0, (T)0), am = mk((T)0, (T)0);
         for (int k = 0; k < S.n_pulse; ++k) {
             if (!S.tetm) {
-                ap = cadd(ap, cmul(smul(rmul(S.ohb, S.dt), S.pulse[0][pi + k * S.plane]), S.amp_pulse[k]));
+                ap = cadd(ap, cmul(smul(rmul(S.ohb, S.dt), S.pulse[0][i + k * S.plane]), S.amp_pulse[k]));
             } else {
                 const cx<T> m = smul(S.dt, mk((T)0.0, rdiv((T)-1.0, S.hbs)));
-                ap = cadd(ap, cmul(cmul(m, S.pulse[0][pi + k * S.plane]), S.amp_pulse[k]));
-                am = cadd(am, cmul(cmul(m, S.pulse[1][pi + k * S.plane]), S.amp_pulse[k]));
+                ap = cadd(ap, cmul(cmul(m, S.pulse[0][i + k * S.plane]), S.amp_pulse[k]));
+                am = cadd(am, cmul(cmul(m, S.pulse[1][i + k * S.plane]), S.amp_pulse[k]));
             }
         }
         if (S.noise.on) {
+            const unsigned r = (unsigned)i / (unsigned)S.N_c, c = (unsigned)i - r * (unsigned)S.N_c;
             const cx<T> xi = noise_xi(S.noise, noise_point((int)r, (int)c, S.N_r, S.N_c, S.periodic_x, S.periodic_y), S.noise_amp);
-            const T nrp = S.res ? (!S.tetm ? rvp[pi] : brvp[pi]) : (T)0;
+            const T nrp = S.res ? (!S.tetm ? rvp[i] : brvp[i]) : (T)0;
             const T scp = rsqrt_rn(rdiv(radd(rmul(S.R, nrp), S.gamma_c), rmul((T)4.0, S.dV)));
             ap = cadd(ap, mk(rmul(xi.re, scp), rmul(xi.im, scp)));
             if (S.tetm) {
-                const T scm = rsqrt_rn(rdiv(radd(rmul(S.R, brvm[pi]), S.gamma_c), rmul((T)4.0, S.dV)));
+                const T scm = rsqrt_rn(rdiv(radd(rmul(S.R, brvm[i]), S.gamma_c), rmul((T)4.0, S.dV)));
                 am = cadd(am, mk(rmul(xi.re, scm), rmul(xi.im, scm)));
             }
         }
-        psip[pi] = cadd(fp[w], ap);
-        if (S.tetm) psim[pi] = cadd(fm[w], am);
-        else if (S.res) rvp[pi] = brvp[pi];
+        psip[i] = cadd(psip[i], ap);
+        if (S.tetm) psim[i] = cadd(psim[i], am);
+        else if (S.res) rvp[i] = brvp[i];
     }
 }
 

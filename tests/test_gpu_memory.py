@@ -12,15 +12,15 @@ PLANE = -(-(N_C + 16) // 32) * 32 * (N_R + 16)
 NOISE = dict(stochastic_amplitude=1e-3)
 # Planes of psi (two reals a point) and n, and of the inputs (pump, potential: one real;
 # pulse: two).  State, two stage planes and an accumulator; the plain scalar
-# iteration also has a second state plane.  SSFM: state and stage planes, its two
-# transformed copies and the table of factors.
+# iteration also has a second state plane.  SSFM: state and stage planes and the
+# table of factors.
 INPUTS = 1 + 1 + 2
 KINDS = {
     "scalar": (dict(), 5 * 3 + INPUTS),
     "scalar_noise": (NOISE, 4 * 3 + INPUTS),
     "spinor": (dict(use_twin_mode=True), 2 * (4 * 3 + INPUTS)),
     "spinor_noise": (dict(use_twin_mode=True, **NOISE), 2 * (4 * 3 + INPUTS)),
-    "ssfm": (dict(iterator="SSFM"), 3 * 3 + INPUTS + 3 * 2),
+    "ssfm": (dict(iterator="SSFM"), 3 * 3 + INPUTS + 2),
 }
 
 
