@@ -29,8 +29,9 @@ void AdjMarch<T>::launch(const AdjFusedParams<T>& Q, int sm_count, cudaStream_t 
     M.strips = (Q.N_c + kMarchOut - 1) / kMarchOut;
     const std::array<int, 4> plan = {Q.N_r, Q.N_c, per_sm, sm_count};
     if (plan != plan_) {
-        plan_rows_ = march_seg_rows<T>(
-            Q.N_r, [&](int L) { return (long long)M.strips * ((Q.N_r + L - 1) / L); }, per_sm, sm_count);
+        plan_rows_ = march_segments(Q.N_r, [&](int L) { return (long long)M.strips * ((Q.N_r + L - 1) / L); }, per_sm,
+                                    sm_count, kMarchCost<T>)
+                         .rows;
         plan_ = plan;
     }
     M.seg_rows = plan_rows_;

@@ -66,8 +66,9 @@ void MarchLauncher<T>::launch(const FusedParams<T>& F, const MarchOptions& o, in
     Q.strips = (F.N_c + kMarchOut - 1) / kMarchOut;
     const std::array<int, 4> plan = {F.N_r, F.N_c, per_sm, sm_count};
     if (plan != plan_) {
-        plan_rows_ = march_seg_rows<T>(
-            F.N_r, [&](int L) { return (long long)Q.strips * ((F.N_r + L - 1) / L); }, per_sm, sm_count);
+        plan_rows_ = march_segments(F.N_r, [&](int L) { return (long long)Q.strips * ((F.N_r + L - 1) / L); }, per_sm,
+                                    sm_count, kMarchCost<T>)
+                         .rows;
         plan_ = plan;
     }
     Q.seg_rows = plan_rows_;
@@ -105,14 +106,15 @@ void MarchBatch<T>::build(const std::vector<FusedParams<T>>& f, bool res, bool f
     if (!kern) pick(std::false_type{}, std::false_type{});
     const int per_sm = march_occupancy(kern, MarchLayout<T>::bytes);
     auto strips = [&](int i) { return (f[2 * i].N_c + kMarchOut - 1) / kMarchOut; };
-    const int L = march_seg_rows<T>(
-        max_rows,
-        [&](int l) {
-            long long items = 0;
-            for (int i = 0; i < n; ++i) items += (long long)strips(i) * ((f[2 * i].N_r + l - 1) / l);
-            return items;
-        },
-        per_sm, sm_count);
+    const int L = march_segments(
+                      max_rows,
+                      [&](int l) {
+                          long long items = 0;
+                          for (int i = 0; i < n; ++i) items += (long long)strips(i) * ((f[2 * i].N_r + l - 1) / l);
+                          return items;
+                      },
+                      per_sm, sm_count, kMarchCost<T>)
+                      .rows;
     std::vector<MarchItem> items;
     for (int i = 0; i < n; ++i) {
         const int rows = f[2 * i].N_r, segs = (rows + L - 1) / L, per = (rows + segs - 1) / segs;

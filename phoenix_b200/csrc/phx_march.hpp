@@ -3,6 +3,7 @@
 #pragma once
 
 #include <array>
+#include <cstdlib>
 #include <map>
 #include <vector>
 
@@ -61,7 +62,8 @@ template <typename T>
 class MarchGeneral {
 public:
     // st: the parameters of the four stages (scalar model: .p only); state
-    // planes per component.  False when no variant takes this iteration.
+    // planes per component.  False when no variant takes this iteration or the
+    // tile kernels are the faster ones for the grid.
     bool launch(const TetmParams<T> (&st)[4], int comps, bool res, const cx<T>* const* psi0, const T* const* n0,
                 cx<T>* const* psi1, T* const* n1, int sm_count, cudaStream_t stream, bool pdl);
 
@@ -71,7 +73,13 @@ private:
                       T* const* n1, int sm_count, cudaStream_t stream, bool pdl);
     std::map<const void*, int> per_sm_;  // CTAs per SM of the kernel variants used so far
     std::array<int, 4> plan_{};          // grid, CTAs per SM and SMs of the last row segmentation
-    int plan_rows_ = 0;
+    int plan_rows_ = 0;                  // 0: the tile kernel
+    // PHX_GENERAL_MARCH: 1 the marching kernel on every grid (an error where no
+    // variant takes the iteration), 0 never; otherwise the faster of the two
+    int forced_ = [] {
+        const char* e = std::getenv("PHX_GENERAL_MARCH");
+        return e && (e[0] == '0' || e[0] == '1') ? e[0] - '0' : -1;
+    }();
 };
 
 // The adjoint's four vector-Jacobian stages of one iteration

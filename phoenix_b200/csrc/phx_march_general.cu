@@ -40,6 +40,42 @@ void take_rest(const Variant& v, GeneralKernel<T, COMPS>& k, int& bytes) {
     take_noise<T, COMPS, NP, 1, 1>(v, k, bytes);
 }
 
+// Marching or tile kernel?  Small grids give every scheduler of the marching
+// kernel less than one warp, whose steps then run at their latency, narrow ones
+// fill half a strip, and long steps of noisy spinors hide nothing behind each
+// other; tiles spread such grids wider.  Both are estimated in us.  The marching
+// kernel: MarchCost as measured on 224 columns with segments of 8 to 32 rows, one
+// to three CTAs per SM.  The tile kernels (phx_step_tetm_fused.cuh): first + round n
+// for n = ceil(tiles / SMs), within 9 % of 45 grids from n = 2 on, and at least
+// `one`.  march_input and tile_input are the shares that a potential or a pulse
+// adds.  Over 896 grids and kinds, from 8 to 1024 columns, the choice costs 5 % at
+// most against the faster of the two.
+// Tile / marching kernel, us: FP32 with a pulse 7.3 / 5.4 at 64^2, 28 / 15 at 768^2;
+// with noise 8.7 / 12.5 at 256^2, 20.2 / 19.4 at 544 x 520, 61 / 40 at 1024^2; the
+// spinor 11.2 / 11.7 at 256^2, 14.9 / 16.4 at 24 x 4096, 27 / 19 at 512^2, with noise
+// 15 / 28 at 256^2, 38 / 45 at 544 x 520, 124 / 74 at 1024^2, with a pulse and a
+// potential as well (one CTA per SM) 98 / 108 at 768^2, 176 / 172 at 1024^2; FP64 with
+// a pulse 13.9 / 14.5 at 384^2, 24 / 28 at 64 x 4096, 50 / 29 at 768^2.
+struct Kind {
+    MarchCost march;
+    double march_input;
+    double one, first, round, tile_input;
+};
+template <typename T>
+const Kind& kind_of(int comps, bool noise) {
+    static const Kind f32[4] = {{{2.0, 6.0, {0.456, 0.722, 1.11}}, 0.09, 6.2, 2.4, 2.7, 0.16},
+                                {{2.4, 6.0, {1.15, 1.61, 2.17}}, 0.04, 8.7, 3.2, 4.2, 0.13},
+                                {{2.0, 6.0, {1.08, 1.77, 2.66}}, 0.10, 11.1, 1.4, 6.6, 0.20},
+                                {{3.2, 6.0, {2.73, 3.12, 4.68}}, 0.25, 14.8, 2.5, 8.9, 0.17}};
+    static const Kind f64[2] = {{{3.3, 6.0, {0.85, 1.47, 2.21}}, 0.20, 5.7, 1.6, 2.6, 0.19},
+                                {{3.3, 6.0, {1.65, 2.45, 3.68}}, 0.07, 8.6, 1.8, 4.4, 0.11}};
+    if (sizeof(T) == 4) return f32[(comps - 1) * 2 + noise];
+    return f64[noise];
+}
+constexpr int kTileW = 32;  // the tile kernels' tiles (go_general, go_tetm_fused)
+template <typename T>
+constexpr int kTileH = sizeof(T) == 4 ? 16 : 8;
+
 }  // namespace
 
 template <typename T>
@@ -55,6 +91,22 @@ bool MarchGeneral<T>::launch_comps(const TetmParams<T> (&st)[4], const cx<T>* co
     if (!kern) return false;
     int& per_sm = per_sm_[reinterpret_cast<const void*>(kern)];
     if (!per_sm) per_sm = march_occupancy(kern, bytes);
+    const int strips = (P.N_c + kMarchOut - 1) / kMarchOut;
+    const std::array<int, 4> plan = {P.N_r, P.N_c, per_sm, sm_count};
+    if (plan != plan_) {
+        const Kind& k = kind_of<T>(COMPS, v.noise);
+        const int inputs = v.nv + v.nq;
+        MarchCost cost = k.march;
+        // (periodic images, FP64 odd widths: 29.7 us a launch at 64 x 4096, 32.4 at 63)
+        for (double& c : cost.step) c *= (1.0 + k.march_input * inputs) * (v.img ? 1.09 : 1.0);
+        const MarchSegments seg = march_segments(
+            P.N_r, [&](int L) { return (long long)strips * ((P.N_r + L - 1) / L); }, per_sm, sm_count, cost);
+        const long long tiles = (long long)((P.N_c + kTileW - 1) / kTileW) * ((P.N_r + kTileH<T> - 1) / kTileH<T>);
+        const double tile_us = std::max(k.one, k.first + k.round * (double)((tiles + sm_count - 1) / sm_count));
+        plan_rows_ = forced_ == 1 || seg.us < tile_us * (1.0 + k.tile_input * inputs) ? seg.rows : 0;
+        plan_ = plan;
+    }
+    if (!plan_rows_) return false;
     MarchGeneralParams<T, COMPS> G;
     for (int s = 0; s < 4; ++s) G.st[s] = st[s];
     for (int q = 0; q < COMPS; ++q) {
@@ -63,13 +115,7 @@ bool MarchGeneral<T>::launch_comps(const TetmParams<T> (&st)[4], const cx<T>* co
         G.psi1[q] = psi1[q];
         G.n1[q] = n1[q];
     }
-    G.strips = (P.N_c + kMarchOut - 1) / kMarchOut;
-    const std::array<int, 4> plan = {P.N_r, P.N_c, per_sm, sm_count};
-    if (plan != plan_) {
-        plan_rows_ = march_seg_rows<T>(
-            P.N_r, [&](int L) { return (long long)G.strips * ((P.N_r + L - 1) / L); }, per_sm, sm_count);
-        plan_ = plan;
-    }
+    G.strips = strips;
     G.seg_rows = plan_rows_;
     G.n_items = G.strips * ((P.N_r + G.seg_rows - 1) / G.seg_rows);
     march_launch(kern, G, G.n_items, bytes, stream, pdl);
@@ -79,26 +125,22 @@ bool MarchGeneral<T>::launch_comps(const TetmParams<T> (&st)[4], const cx<T>* co
 template <typename T>
 bool MarchGeneral<T>::launch(const TetmParams<T> (&st)[4], int comps, bool res, const cx<T>* const* psi0, const T* const* n0,
                              cx<T>* const* psi1, T* const* n1, int sm_count, cudaStream_t stream, bool pdl) {
+    if (forced_ == 0) return false;
     const StageParams<T>& P = st[0].p;
-    // Small grids give every scheduler less than one warp, whose steps then run at
-    // their latency; the tile kernels spread such a grid wider.  us per iteration,
-    // tiles against march: FP32 without noise 9.2 / 7.8 at 128^2 already; with
-    // noise (long steps) 10.2 / 14.4 at 256^2, 22.7 / 23.3 at 512^2, 68.9 / 46.5 at
-    // 1024^2, the spinor 28 / 46 at 384^2, 48 / 46 at 512^2; FP64 9.1 / 14.3 at
-    // 256^2, 16.4 / 16.7 at 384^2, 28.6 / 21.8 at 512^2.
-    const long long points = (long long)P.N_r * P.N_c;
-    if (points < (P.noise.on ? 280000 : (sizeof(T) == 8 ? 150000 : 0))) return false;
     // 32-bit indices over every group's planes; a reservoir with its pump; real
     // potential coefficients
     const int groups = std::max({1, P.n_pump, P.n_pot, P.n_pulse});
-    if (!res || P.n_pump < 1 || P.plane * groups >= (1LL << 31)) return false;
+    bool takes = res && P.n_pump >= 1 && P.plane * groups < (1LL << 31);
     for (int s = 0; s < 4; ++s)
-        for (int g = 0; g < P.n_pot; ++g)
-            if (st[s].p.pot_c[g].im != (T)0) return false;
-    if (comps == 1) return launch_comps<1>(st, psi0, n0, psi1, n1, sm_count, stream, pdl);
+        for (int g = 0; g < P.n_pot; ++g) takes = takes && st[s].p.pot_c[g].im == (T)0;
+    bool done = false;
+    if (takes && comps == 1) done = launch_comps<1>(st, psi0, n0, psi1, n1, sm_count, stream, pdl);
     // FP64: two polarisations' rows do not fit the registers
-    if constexpr (sizeof(T) == 4) return launch_comps<2>(st, psi0, n0, psi1, n1, sm_count, stream, pdl);
-    return false;
+    if constexpr (sizeof(T) == 4) {
+        if (takes && comps == 2) done = launch_comps<2>(st, psi0, n0, psi1, n1, sm_count, stream, pdl);
+    }
+    if (!done && forced_ == 1) fail(PHX_ERR_UNSUPPORTED, "no marching kernel takes this iteration (PHX_GENERAL_MARCH=1)");
+    return done;
 }
 
 template class MarchGeneral<float>;

@@ -9,32 +9,38 @@
 
 namespace phx {
 
-// Rows per segment.  A segment of L rows costs about L + extra full steps (its
-// first rows run through some stages only; four stages: 3), and an SM with w
-// CTAs takes cost(w) per step of all of them (measured at 1024^2; one CTA
-// leaves its schedulers waiting on one warp's latencies).  More CTAs than fit
-// at once run in rounds.  4096^2 FP32: 184 us at 64 rows (estimate 189), 196 at
-// 32 (199).
+// What a launch of a marching kernel takes: base + (L + extra) step(w) for
+// segments of L rows with w CTAs on an SM.  A segment runs L + 6 steps, `extra`
+// counts them in full ones (its first rows go through some of the stages only);
+// one CTA leaves its schedulers waiting on one warp's latencies, so a step of two
+// CTAs does not take twice its time.  More CTAs than fit at once run in rounds.
+struct MarchCost {
+    double base, extra, step[3];  // us; step: with one, two, three CTAs per SM
+    double of(int ctas) const { return ctas <= 0 ? 0.0 : (ctas <= 3 ? step[ctas - 1] : step[2] * ctas / 3); }
+};
+// The plain scalar iteration at 1024^2 (no base: its own segments are all that it
+// is used to compare); 4096^2 FP32: 184 us at 64 rows (estimate 189), 196 at 32
+// (199).  The adjoint's kernel takes the same figures; its steps last longer and
+// its start is nearer four of them.
 template <typename T>
-double march_cost(int L, long long items, int per_sm, int sm_count, double extra) {
-    const double cost32[4] = {0.0, 0.47, 0.74, 1.05}, cost64[3] = {0.0, 0.92, 1.52};
-    auto cost = [&](int w) {
-        if (sizeof(T) == 4) return w <= 3 ? cost32[w] : cost32[3] * w / 3;
-        return w <= 2 ? cost64[w] : cost64[2] * w / 2;
-    };
-    const long long ctas = (items + kMarchWarps - 1) / kMarchWarps, w = (ctas + sm_count - 1) / sm_count;
-    return (L + extra) * ((double)(w / per_sm) * cost(per_sm) + cost((int)(w % per_sm)));
-}
-// the cheapest segment length of at most max_rows, items(L) segments in all
-template <typename T, typename Items>
-int march_seg_rows(int max_rows, const Items& items, int per_sm, int sm_count, double extra = 3.0) {
-    int best_L = max_rows;
-    double best = -1.0;
+constexpr MarchCost kMarchCost = sizeof(T) == 4 ? MarchCost{0.0, 3.0, {0.47, 0.74, 1.05}}
+                                                : MarchCost{0.0, 3.0, {0.92, 1.52, 2.28}};
+
+// the cheapest segment length of at most max_rows, items(L) segments in all, and its time
+struct MarchSegments {
+    int rows;
+    double us;
+};
+template <typename Items>
+MarchSegments march_segments(int max_rows, const Items& items, int per_sm, int sm_count, const MarchCost& cost) {
+    MarchSegments best{max_rows, -1.0};
     for (int L = std::min(max_rows, 2); L <= std::min(max_rows, 256); ++L) {
-        const double t = march_cost<T>(L, items(L), per_sm, sm_count, extra);
-        if (best < 0.0 || t < best) best = t, best_L = L;
+        const long long ctas = (items(L) + kMarchWarps - 1) / kMarchWarps, w = (ctas + sm_count - 1) / sm_count;
+        const double us =
+            cost.base + (L + cost.extra) * ((double)(w / per_sm) * cost.of(per_sm) + cost.of((int)(w % per_sm)));
+        if (best.us < 0.0 || us < best.us) best = {L, us};
     }
-    return best_L;
+    return best;
 }
 template <typename K, typename Q>
 void march_launch(K kern, const Q& params, int n_items, int bytes, cudaStream_t stream, bool pdl) {

@@ -69,29 +69,37 @@ def test_fma_arithmetic(require_gpu, monkeypatch, res, pot, temporal):
         np.testing.assert_array_equal(x, y)
 
 
-def general(n_c, n_r, dtype, px, py, monkeypatch, staged, tetm=False, pumps=1, pot=1, pulse=0, dw=0.0, iters=4):
+def general(n_c, n_r, dtype, px, py, monkeypatch, staged, tetm=False, pumps=1, pot=1, pulse=0, dw=0.0, iters=4, march=None,
+            cell=1.0, plant=()):
+    """march: PHX_GENERAL_MARCH (by default the rule between the marching and the tile
+    kernels); plant: (field, row, column, value) set in the first group of the inputs."""
     monkeypatch.setenv("PHX_TETM_FUSED", "0" if staged else "1")
     monkeypatch.setenv("PHX_GENERAL_FUSED", "0" if staged else "1")
+    if march is None:
+        monkeypatch.delenv("PHX_GENERAL_MARCH", raising=False)
+    else:
+        monkeypatch.setenv("PHX_GENERAL_MARCH", march)
     T = pb.Temporal
     rng = np.random.default_rng([n_c, n_r, 3])
-    sp = pb.SystemParameters(N_c=n_c, N_r=n_r, L_x=0.3 * n_c, L_y=0.2 * n_r, h_bar_s=0.6582, m_eff=0.5, gamma_c=0.2,
+    sp = pb.SystemParameters(N_c=n_c, N_r=n_r, L_x=0.3 * n_c * cell, L_y=0.2 * n_r * cell, h_bar_s=0.6582, m_eff=0.5, gamma_c=0.2,
                              gamma_r=0.3, g_c=0.05, g_r=0.08, R=0.04, g_pm=-0.01, delta_LT=0.3, use_twin_mode=tetm,
-                             periodic_boundary_x=px, periodic_boundary_y=py, dtype=dtype, dt=0.002, t_max=1e12,
+                             periodic_boundary_x=px, periodic_boundary_y=py, dtype=dtype, dt=0.002 * cell ** 2, t_max=1e12,
                              fft_every=1e12, pump_temporal=[T(), T("cos", 0.004, 0.01, 200.0)][:pumps],
-                             potential_temporal=[T("gauss", 0.004, 0.01, 1.0)][:pot],
-                             pulse_temporal=[T("iexp", 0.004, 0.01, 50.0)][:pulse], stochastic_amplitude=dw, random_seed=11)
+                             potential_temporal=[T("gauss", 0.004, 0.01, 1.0)] * pot,
+                             pulse_temporal=[T("iexp", 0.004, 0.01, 50.0)] * pulse, stochastic_amplitude=dw, random_seed=11)
     comps = ("plus", "minus") if tetm else ("plus",)
     with pb.Solver(sp) as s:
         for c in comps:
             z = lambda: rng.standard_normal((n_r, n_c)) + 1j * rng.standard_normal((n_r, n_c))  # noqa: E731
-            s.set_field("psi_" + c, z())
-            s.set_field("n_" + c, rng.random((n_r, n_c)))
-            for g in range(pumps):
-                s.set_field("pump_" + c, 3.0 * rng.random((n_r, n_c)), g)
-            for g in range(pot):
-                s.set_field("potential_" + c, 0.3 * rng.standard_normal((n_r, n_c)), g)
-            for g in range(pulse):
-                s.set_field("pulse_" + c, z(), g)
+            f = {("psi_", 0): z(), ("n_", 0): rng.random((n_r, n_c))}
+            f.update({("pump_", g): 3.0 * rng.random((n_r, n_c)) for g in range(pumps)})
+            f.update({("potential_", g): 0.3 * rng.standard_normal((n_r, n_c)) for g in range(pot)})
+            f.update({("pulse_", g): z() for g in range(pulse)})
+            for name, row, col, value in plant:
+                if (name, 0) in f:
+                    f[name, 0][row, col] = value
+            for (name, g), v in f.items():
+                s.set_field(name + c, v, g)
         info = s.run(iters)
         assert staged == (info.kernel_launches >= 4 * iters)
         return [s.get_field(f + c) for c in comps for f in ("psi_", "n_")]
@@ -106,14 +114,33 @@ INPUTS = [(1, 1, 0, 0.02), (1, 0, 0, 0.02), (1, 1, 1, 0.0), (1, 0, 1, 0.02), (2,
                          [(False, d) + i for d in ("f32", "f64") for i in INPUTS] +
                          [(True, d) + i for d in ("f32", "f64") for i in INPUTS + [(1, 1, 0, 0.0)]])
 def test_general_and_spinor_iterations(require_gpu, monkeypatch, tetm, dtype, pumps, pot, pulse, dw):
-    sizes = [(8, 8, True, True), (56, 13, True, False), (114, 61, False, True)]
-    if dw > 0 or dtype == "f64":  # below 280000 points these run the tile kernels: the same widths, taller
-        sizes = [(8, 35001, True, True), (56, 5003, True, False), (114, 2461, False, True)]
-    if dtype == "f64":
-        sizes.append((57, 4913, False, False))
+    sizes = [(8, 8, True, True), (56, 13, True, False), (114, 61, False, True), (114, 2461, True, True)]
+    if dtype == "f64":  # odd widths: periodic images (with walls in x there are none)
+        sizes += [(57, 49, False, False), (57, 33, True, True), (113, 40, True, False), (9, 8, True, True)]
+    # the marching kernel whatever the grid, an error where it has no variant: FP64
+    # spinors and spinors with two pump groups run the tile kernel
+    march = "0" if tetm and (dtype == "f64" or pumps > 1) else "1"
     for n_c, n_r, px, py in sizes:
         want = general(n_c, n_r, dtype, px, py, monkeypatch, True, tetm, pumps, pot, pulse, dw)
-        got = general(n_c, n_r, dtype, px, py, monkeypatch, False, tetm, pumps, pot, pulse, dw)
+        got = general(n_c, n_r, dtype, px, py, monkeypatch, False, tetm, pumps, pot, pulse, dw, march=march)
+        for x, y in zip(got, want):
+            np.testing.assert_array_equal(x, y, err_msg=f"{n_c} x {n_r}")
+
+
+def test_forced_marching_kernel_refuses_what_it_has_no_variant_for(require_gpu, monkeypatch):
+    with pytest.raises(pb.PhxError, match="PHX_GENERAL_MARCH"):
+        general(56, 13, "f32", True, True, monkeypatch, False, pot=1, pulse=2, march="1")
+
+
+# the rule between the marching and the tile kernels, on grids of either side: one
+# tile, narrow and long, one round of tiles and several
+@pytest.mark.parametrize("tetm,dtype,pot,pulse,dw", [(False, "f32", 1, 1, 0.0), (False, "f32", 0, 0, 0.02),
+                                                     (True, "f32", 1, 0, 0.0), (True, "f32", 1, 1, 0.02),
+                                                     (False, "f64", 0, 1, 0.0), (False, "f64", 1, 0, 0.02)])
+def test_general_iterations_as_dispatched(require_gpu, monkeypatch, tetm, dtype, pot, pulse, dw):
+    for n_c, n_r in [(8, 8), (24, 700), (64, 1000), (500, 444), (768, 770)]:
+        want = general(n_c, n_r, dtype, True, False, monkeypatch, True, tetm, 1, pot, pulse, dw, iters=2)
+        got = general(n_c, n_r, dtype, True, False, monkeypatch, False, tetm, 1, pot, pulse, dw, iters=2)
         for x, y in zip(got, want):
             np.testing.assert_array_equal(x, y, err_msg=f"{n_c} x {n_r}")
 
