@@ -162,14 +162,20 @@ __device__ __forceinline__ cx<T> shfl_dn1(cx<T> z) {
 // Muller, Raina, "Accelerating correctly rounded floating-point division when
 // the divisor is known in advance", IEEE Trans. Comput. 53(8), 2004).  It holds
 // while the residual does not underflow, in FP32 for |x| > 2^-100; below that
-// the last bit may differ, and an exact zero may change its sign.
-__device__ __forceinline__ float div_known(float x, float y, float z) {
-    const float q = __fmul_rn(x, z);
-    return __fmaf_rn(__fmaf_rn(-q, y, x), z, q);
+// the last bit may differ, and an exact zero may change its sign.  A quotient
+// within two last places of the largest finite number may come out infinite.
+// For an infinite x, or one whose quotient overflows, the residual is not a
+// number: the quotient then is x z (div_known), or not a number either
+// (div_known_finite, where no use of an infinite quotient is left).
+template <typename T>
+__device__ __forceinline__ T div_known_finite(T x, T y, T z) {
+    const T q = rmul(x, z);
+    return rfma(rfma(-q, y, x), z, q);
 }
-__device__ __forceinline__ double div_known(double x, double y, double z) {
-    const double q = __dmul_rn(x, z);
-    return __fma_rn(__fma_rn(-q, y, x), z, q);
+template <typename T>
+__device__ __forceinline__ T div_known(T x, T y, T z) {
+    const T r = div_known_finite(x, y, z);
+    return r == r ? r : rmul(x, z);
 }
 
 // (one_over_h_bar_s g_c) (-i psi) / dV: the stochastic drift of psi
@@ -188,7 +194,10 @@ struct ScalarGlobalSrc {
     __device__ __forceinline__ int n_pot() const { return P.n_pot; }
     __device__ __forceinline__ int n_pulse() const { return P.n_pulse; }
     __device__ __forceinline__ bool noise() const { return P.noise.on != 0; }
-    // real_pot: every potential coefficient is known to be real
+    // real_pot: every potential coefficient is known to be real; the products with
+    // its and the reservoir's zero imaginary part are left out.  That changes the
+    // sign of an exact zero, and where psi or the potential is not finite, 0 times
+    // infinity, a NaN, is missing from results that are infinite anyway.
     static __device__ __forceinline__ constexpr bool real_pot() { return false; }
     static __device__ __forceinline__ T over_dV(const StageParams<T>& S, T x) { return rdiv(x, S.dV); }
     __device__ __forceinline__ T pump(int g) const { return __ldg(P.pump + idx + g * P.plane); }
@@ -208,11 +217,14 @@ __device__ __forceinline__ void rhs_scalar_src(const StageParams<T>& P, const Sr
     wf = cadd(wf, smul(rmul(P.ohb_gc, in_psi_norm), in_wf_mi));
     wf = csub(wf, smul(P.half_gamma_c, in_wf));
     if constexpr (RES) {
-        // the reference's complex products with a reservoir of imaginary part
-        // zero, less the products with that zero (only the sign of an exact
-        // zero could tell)
-        wf = cadd(wf, smul(rmul(P.ohb_gr, in_rv), in_wf_mi));
-        wf = cadd(wf, smul(rmul(P.half_R, in_rv), in_wf));
+        if constexpr (Src::real_pot()) {
+            wf = cadd(wf, smul(rmul(P.ohb_gr, in_rv), in_wf_mi));
+            wf = cadd(wf, smul(rmul(P.half_R, in_rv), in_wf));
+        } else {
+            const cx<T> rv = mk(in_rv, (T)0);
+            wf = cadd(wf, cmul(smul(P.ohb_gr, rv), in_wf_mi));
+            wf = cadd(wf, cmul(smul(P.half_R, rv), in_wf));
+        }
         const T s = -radd(P.gamma_r, rmul(P.R, in_psi_norm));
         T krv = rmul(s, in_rv);
         for (int g = 0; g < src.n_pump(); ++g) krv = radd(krv, rmul(src.pump(g), P.pump_c[g].re));
@@ -220,8 +232,8 @@ __device__ __forceinline__ void rhs_scalar_src(const StageParams<T>& P, const Sr
     }
     for (int g = 0; g < src.n_pot(); ++g) {
         const T v = src.pot(g);
-        wf = cadd(wf, src.real_pot() ? smul(rmul(P.ohb, rmul(v, P.pot_c[g].re)), in_wf_mi)
-                                     : cmul(smul(P.ohb, smul(v, P.pot_c[g])), in_wf_mi));
+        wf = cadd(wf, Src::real_pot() ? smul(rmul(P.ohb, rmul(v, P.pot_c[g].re)), in_wf_mi)
+                                      : cmul(smul(P.ohb, smul(v, P.pot_c[g])), in_wf_mi));
     }
     for (int g = 0; g < src.n_pulse(); ++g) wf = cadd(wf, cmul(smul(P.ohb, src.pulse(g)), P.pulse_c[g]));
     if (src.noise()) {

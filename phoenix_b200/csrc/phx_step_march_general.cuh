@@ -6,14 +6,18 @@
 //
 // The numbers of groups, the noise and the kind of the potential's coefficient
 // are template parameters, so a step is one straight run of instructions; the
-// host takes the kernel where a variant and its ring fit (phx_march.cu) and the
-// tile kernels (phx_step_tetm_fused.cuh) elsewhere.
+// host takes the kernel where a variant and its ring fit and it is the faster one
+// (phx_march_general.cu), and the tile kernels (phx_step_tetm_fused.cuh) elsewhere.
 //
 // The noise value of a point and its scale are drawn once, when the first
 // stage meets the row, and kept in the ring for the other three.
 //
 // Per point the operations are rhs_scalar_src's / rhs_tetm_src's and the kRk4*
-// sums of the stage kernels, in the same order (bit-identical results).
+// sums of the stage kernels, in the same order: bit-identical results, but for the
+// sign of an exact zero and for divisions by dV outside div_known's range (FP32
+// dividends below 2^-100: their last bit).  A value that is not finite in the
+// stage kernels is not finite here; it may be infinite where theirs is NaN
+// (ScalarGlobalSrc::real_pot).
 #pragma once
 
 #include "phx_stage_tetm.cuh"
@@ -64,7 +68,10 @@ struct MarchSrc {
     static __device__ __forceinline__ constexpr int n_pulse() { return NQ; }
     static __device__ __forceinline__ constexpr bool noise() { return NOISE; }
     static __device__ __forceinline__ constexpr bool real_pot() { return REALV; }
-    static __device__ __forceinline__ T over_dV(const StageParams<T>& S, T x) { return div_known(x, S.dV, S.inv_dV); }
+    // the drift of an infinite psi is taken from the infinity of its |psi|^2, the
+    // reservoir's gain from an infinite n added to the opposite infinity of its
+    // loss: NaN whatever the quotient
+    static __device__ __forceinline__ T over_dV(const StageParams<T>& S, T x) { return div_known_finite(x, S.dV, S.inv_dV); }
     __device__ __forceinline__ T pump(int c, int g) const { return pu[g][c][j]; }
     __device__ __forceinline__ T pot(int c, int g) const { return po[g][c][j]; }
     __device__ __forceinline__ cx<T> pulse(int c, int g) const { return ps[g][c][j]; }

@@ -145,3 +145,23 @@ def test_a_new_handle_does_not_read_what_its_error_flag_held_before(require_gpu,
             s.set_field_tensor("psi_plus", psi_t)
             s.run(50)
             assert torch.isfinite(torch.view_as_real(s.get_field_tensor("psi_plus"))).all()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+def test_an_infinite_component_leaves_no_number_behind(require_gpu, dtype):
+    """The reference multiplies psi by the complex reservoir, whose imaginary part is
+    zero: 0 times infinity makes both components NaN within one stage (Newton has one)."""
+    n = 32
+    rng = np.random.default_rng(1)
+    psi = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    psi[5, 7] = complex(np.inf, 0.5)
+    psi[20, 9] = complex(0.5, -np.inf)
+    with pb.Solver(_system(n, iterator="Newton", dtype=dtype, dt=1e-3)) as s:
+        s.set_field("psi_plus", psi)
+        s.set_field("n_plus", rng.random((n, n)))
+        s.set_field("pump_plus", rng.random((n, n)))
+        s.run(1)
+        out = s.get_field("psi_plus")
+    for r, c in ((5, 7), (20, 9)):
+        assert np.isnan(out[r, c].real) and np.isnan(out[r, c].imag)
+    assert np.isfinite(out).sum() == n * n - 2 * 5  # the points and their four neighbours

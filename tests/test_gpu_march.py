@@ -132,6 +132,28 @@ def test_forced_marching_kernel_refuses_what_it_has_no_variant_for(require_gpu, 
         general(56, 13, "f32", True, True, monkeypatch, False, pot=1, pulse=2, march="1")
 
 
+# a run that diverges, from any input and from operations that overflow (|psi|^2,
+# R n / dV): not finite where the stage kernels are not, the same values elsewhere
+@pytest.mark.parametrize("tetm,dtype,pumps,pot,pulse,dw", [(False, "f32", 1, 1, 1, 0.02), (False, "f32", 2, 0, 0, 0.0),
+                                                           (False, "f32", 1, 1, 1, 0.0), (True, "f32", 1, 1, 0, 0.02),
+                                                           (True, "f32", 1, 1, 0, 0.0), (False, "f64", 1, 1, 0, 0.02),
+                                                           (False, "f64", 2, 1, 1, 0.0)])
+def test_values_that_are_not_finite(require_gpu, monkeypatch, tetm, dtype, pumps, pot, pulse, dw):
+    inf, huge, big = float("inf"), 1e25 if dtype == "f32" else 1e160, 1e37 if dtype == "f32" else 1e307
+    plant = [("psi_", 0, 0, inf), ("psi_", 20, 30, complex(0.5, -inf)), ("psi_", 20, 60, complex(inf, inf)),
+             ("psi_", 20, 90, huge * (1 - 1j)), ("psi_", 40, 30, complex(float("nan"), 1.0)), ("n_", 40, 60, inf),
+             ("n_", 40, 90, big), ("pump_", 60, 30, inf), ("potential_", 60, 60, inf), ("potential_", 60, 90, -inf)]
+    for iters in (1, 2):
+        args = (114, 80, dtype, True, False, monkeypatch)
+        kind = dict(tetm=tetm, pumps=pumps, pot=pot, pulse=pulse, dw=dw, iters=iters, cell=0.1, plant=plant)
+        want = general(*args, True, **kind)
+        got = general(*args, False, march="1", **kind)
+        assert all(np.isfinite(v).any() and not np.isfinite(v).all() for v in want)
+        for x, y in zip(got, want):
+            np.testing.assert_array_equal(np.isfinite(x), np.isfinite(y))
+            np.testing.assert_array_equal(x[np.isfinite(x)], y[np.isfinite(y)])
+
+
 # the rule between the marching and the tile kernels, on grids of either side: one
 # tile, narrow and long, one round of tiles and several
 @pytest.mark.parametrize("tetm,dtype,pot,pulse,dw", [(False, "f32", 1, 1, 0.0), (False, "f32", 0, 0, 0.02),
