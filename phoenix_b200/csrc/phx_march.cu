@@ -24,16 +24,16 @@ void MarchLauncher<T>::launch(const FusedParams<T>& F, const MarchOptions& o, in
         if (F.pump && F.pump_c[s] != (T)1) unit = false;
         if (F.pot && F.pot_c[s] != (T)1) unit = false;
     }
-    // the variant with temporal coefficients always takes the potential's terms
-    const bool pot = F.pot != nullptr || !unit;
+    const bool pot = F.pot != nullptr;
     K kern = nullptr;
     using std::false_type;
     using std::true_type;
     auto pick = [&](auto res, auto fma, auto img) {
         constexpr bool R = decltype(res)::value, M = decltype(fma)::value, I = decltype(img)::value;
-        kern = !pot ? (K)rk4_march_kernel<T, R, false, true, M, false, I, MINB>
-                    : (unit ? (K)rk4_march_kernel<T, R, true, true, M, false, I, MINB>
-                            : (K)rk4_march_kernel<T, R, true, false, M, false, I, MINB>);
+        kern = pot ? (unit ? (K)rk4_march_kernel<T, R, true, true, M, false, I, MINB>
+                           : (K)rk4_march_kernel<T, R, true, false, M, false, I, MINB>)
+                   : (unit ? (K)rk4_march_kernel<T, R, false, true, M, false, I, MINB>
+                           : (K)rk4_march_kernel<T, R, false, false, M, false, I, MINB>);
     };
     auto pick_store = [&](auto res, auto img) {
         constexpr bool R = decltype(res)::value, I = decltype(img)::value;
@@ -80,21 +80,22 @@ template <typename T>
 void MarchBatch<T>::build(const std::vector<FusedParams<T>>& f, bool res, bool fma, int sm_count, cudaStream_t stream) {
     using K = void (*)(MarchBatchParams<T>);
     constexpr int MINB = kMarchMinB<T>;
-    bool pot = false;
-    int max_rows = 1;
+    int with_pot = 0, max_rows = 1;
     const int n = (int)(f.size() / 2);
     for (int i = 0; i < n; ++i) {
-        pot = pot || f[2 * i].pot != nullptr;
+        with_pot += f[2 * i].pot != nullptr;
         max_rows = std::max(max_rows, f[2 * i].N_r);
     }
     K kern = nullptr;
+    auto pick_pots = [&](auto r, auto m, auto img) {
+        constexpr bool R = decltype(r)::value, M = decltype(m)::value, I = decltype(img)::value;
+        kern = with_pot == 0   ? (K)rk4_march_batch_kernel<T, R, 0, M, I, MINB>
+               : with_pot == n ? (K)rk4_march_batch_kernel<T, R, 1, M, I, MINB>
+                               : (K)rk4_march_batch_kernel<T, R, 2, M, I, MINB>;
+    };
     auto pick = [&](auto m, auto img) {
-        constexpr bool M = decltype(m)::value, I = decltype(img)::value;
-        if (res)
-            kern = pot ? (K)rk4_march_batch_kernel<T, true, true, M, I, MINB> : (K)rk4_march_batch_kernel<T, true, false, M, I, MINB>;
-        else
-            kern = pot ? (K)rk4_march_batch_kernel<T, false, true, M, I, MINB>
-                       : (K)rk4_march_batch_kernel<T, false, false, M, I, MINB>;
+        if (res) pick_pots(std::true_type{}, m, img);
+        else pick_pots(std::false_type{}, m, img);
     };
     images_ = false;
     for (int i = 0; i < n; ++i) images_ = images_ || march_needs_images(f[2 * i].N_c, f[2 * i].img_x);

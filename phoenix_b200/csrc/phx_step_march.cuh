@@ -105,7 +105,8 @@ __device__ __forceinline__ void ring_two(const unsigned char* p, double* v) {
 
 // One warp's segment: rows [R0, R1) of strip `strip`; `ring` is the warp's
 // shared memory.
-// POT: the potential's terms are evaluated (an absent plane counts as zero).
+// POT: there is a potential (where there is none its terms are not evaluated: 0
+// times an infinite psi would not be zero).
 // UNIT: every temporal coefficient is exactly 1 (constant envelopes); the
 // products with it, which change nothing, are left out.  STORE: also write
 // the stage values Y2..Y4 of the stored points, which the adjoint's backward
@@ -125,15 +126,12 @@ __device__ __forceinline__ void march_segment(const FusedParams<T>& P, int strip
     const int lane = threadIdx.x & 31;
     const int c = strip * kMarchOut - 4 + CPT * lane;
     const int pitch = (int)P.pitch;
-    const bool has_pump = RES && P.pump != nullptr, has_pot = POT && P.pot != nullptr;
+    const bool has_pump = RES && P.pump != nullptr;
     unsigned char* const mine = ring + lane * 16;
-    if ((RES && !has_pump) || (POT && !has_pot)) {
+    if (RES && !has_pump) {  // an absent pump counts as zero
         for (int k = 0; k < kMarchRing; ++k)
 #pragma unroll
-            for (int j = 0; j < CPT; ++j) {
-                reinterpret_cast<T*>(mine + k * Lay::row_bytes + Lay::pump_off)[j] = (T)0;
-                reinterpret_cast<T*>(mine + k * Lay::row_bytes + Lay::pot_off)[j] = (T)0;
-            }
+            for (int j = 0; j < CPT; ++j) reinterpret_cast<T*>(mine + k * Lay::row_bytes + Lay::pump_off)[j] = (T)0;
     }
 
     // rows are counted from k = 0 at R0 - 4: step k evaluates stage s (0-based)
@@ -155,9 +153,7 @@ __device__ __forceinline__ void march_segment(const FusedParams<T>& P, int strip
             cp_async<Lay::RB>(d + Lay::n_off, P.n0 + next_g);
             if (has_pump) cp_async<Lay::RB>(d + Lay::pump_off, P.pump + next_g);
         }
-        if constexpr (POT) {
-            if (has_pot) cp_async<Lay::RB>(d + Lay::pot_off, P.pot + next_g);
-        }
+        if constexpr (POT) cp_async<Lay::RB>(d + Lay::pot_off, P.pot + next_g);
         cp_async_commit();
         ++next_k;
         ++next_r;
@@ -348,14 +344,22 @@ struct MarchBatchParams {
     int n_items, dir;
 };
 
-template <typename T, bool RES, bool POT, bool FMA, bool IMG, int MINB>
+// POTS: no instance has a potential (0), all have one (1), or some (2)
+template <typename T, bool RES, int POTS, bool FMA, bool IMG, int MINB>
 __global__ void __launch_bounds__(32 * kMarchWarps, MINB) rk4_march_batch_kernel(const __grid_constant__ MarchBatchParams<T> Q) {
     extern __shared__ __align__(16) unsigned char march_smem[];
     const int warp = threadIdx.x >> 5, item = blockIdx.x * kMarchWarps + warp;
     if (item >= Q.n_items) return;
     const MarchItem it = Q.items[item];
     const FusedParams<T> P = Q.f[2 * it.inst + Q.dir];
-    march_segment<T, RES, POT, true, FMA, false, IMG>(P, it.strip, it.r0, it.r1, march_smem + warp * MarchLayout<T>::warp_bytes);
+    unsigned char* const ring = march_smem + warp * MarchLayout<T>::warp_bytes;
+    if constexpr (POTS != 0) {
+        if (POTS == 1 || P.pot != nullptr) {
+            march_segment<T, RES, true, true, FMA, false, IMG>(P, it.strip, it.r0, it.r1, ring);
+            return;
+        }
+    }
+    if constexpr (POTS != 1) march_segment<T, RES, false, true, FMA, false, IMG>(P, it.strip, it.r0, it.r1, ring);
 }
 
 }  // namespace phx

@@ -112,6 +112,24 @@ def test_every_batch_tile_shape_with_more_tiles_than_ctas(require_gpu, shape, mo
             np.testing.assert_array_equal(b.get_field(i, "n_plus"), np.real(ref["n_plus"]), err_msg=f"instance {i} n")
 
 
+def test_batch_instance_without_a_potential_beside_one_with(require_gpu, monkeypatch):
+    """The marching warps multiply an instance by its own potential only: an infinite
+    psi gives what the tile kernels make of it."""
+    inst = [make_instance(60, 64, 48, "f32"), make_instance(61, 58, 40, "f32", pot=False)]
+    for _, f in inst:
+        f["psi_plus"][10, 20] = complex(np.inf, 1.0)
+    out = {}
+    for shape in (2, 3):
+        monkeypatch.setenv("PHX_BATCH_SHAPE", str(shape))
+        with pb.BatchSolver([pb.system_from_case(c) for c, _ in inst]) as b:
+            for i, (c, f) in enumerate(inst):
+                load_batch(b, i, c, f)
+            b.run(1)
+            out[shape] = [b.get_field(i, name) for i in range(2) for name in ("psi_plus", "n_plus")]
+    for x, y in zip(out[2], out[3]):
+        np.testing.assert_array_equal(x, y)
+
+
 def test_batch_matches_single_solvers_ragged_fp32(require_gpu):
     """Sweep-shaped batch: grid sizes from {128, 256, 512, 1024}, pump 0.8-3.0x
     threshold, disorder 0.05-0.2 meV rms; each instance equals its own Solver."""

@@ -18,7 +18,8 @@ SIZES = [(8, 8), (10, 9), (54, 37), (56, 12), (58, 140), (112, 35), (114, 301), 
 ODD = [(9, 8), (55, 41), (57, 33), (113, 150)]
 
 
-def run(n_c, n_r, dtype, px, py, shape, monkeypatch, res=True, pump=True, pot=True, temporal=False, fma=False, iters=5):
+def run(n_c, n_r, dtype, px, py, shape, monkeypatch, res=True, pump=True, pot=True, temporal=False, fma=False, iters=5,
+        plant=()):
     monkeypatch.setenv("PHX_STAGE_SHAPE", str(shape))
     rng = np.random.default_rng([n_c, n_r])
     T = pb.Temporal
@@ -27,6 +28,8 @@ def run(n_c, n_r, dtype, px, py, shape, monkeypatch, res=True, pump=True, pot=Tr
                              pump_temporal=[T("cos", 0.02, 0.05, 40.0) if temporal else T()] if pump and res else [],
                              potential_temporal=[T("gauss", 0.02, 0.05, 1.0) if temporal else T()] if pot else [], fma=fma)
     psi0 = rng.standard_normal((n_r, n_c)) + 1j * rng.standard_normal((n_r, n_c))
+    for row, col, value in plant:
+        psi0[row, col] = value
     with pb.Solver(sp) as s:
         s.set_field("psi_plus", psi0)
         if res:
@@ -57,6 +60,18 @@ def test_edges_of_strips_and_segments(require_gpu, monkeypatch, dtype, px, py):
 def test_inputs_and_envelopes(require_gpu, monkeypatch, dtype, res, pump, pot, temporal):
     a = run(114, 70, dtype, True, False, 12, monkeypatch, res, pump, pot, temporal)
     b = run(114, 70, dtype, True, False, 2, monkeypatch, res, pump, pot, temporal)
+    for x, y in zip(a, b):
+        np.testing.assert_array_equal(x, y)
+
+
+# without a potential nothing is multiplied by one: an infinite psi gives what the
+# tile kernels (shape 4) make of it
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+@pytest.mark.parametrize("temporal,pot", [(True, False), (False, False), (True, True)])
+def test_infinite_psi(require_gpu, monkeypatch, dtype, temporal, pot):
+    inf = ((10, 20, complex(np.inf, 1.0)), (50, 70, complex(0.0, -np.inf)))
+    a = run(114, 70, dtype, True, False, 12, monkeypatch, True, True, pot, temporal, iters=1, plant=inf)
+    b = run(114, 70, dtype, True, False, 4, monkeypatch, True, True, pot, temporal, iters=1, plant=inf)
     for x, y in zip(a, b):
         np.testing.assert_array_equal(x, y)
 
