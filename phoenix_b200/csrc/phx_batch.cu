@@ -36,23 +36,28 @@ namespace phx {
 // FP64 tiles are half as high (shared memory of the two TMA slots).
 // MINB: CTAs per SM the register allocation leaves room for (the 12-warp
 // shapes run two per SM).
-constexpr int kBatchShapes = 5;
+// The last FP64 shape, 32 x 8 tiles of four warps, is for batches of small
+// grids: us per iteration against the best of the others 6.7 / 7.3 for four
+// instances of 64^2 and for sixteen of 32^2, 7.0 / 8.1 for 64 of 16^2.  In FP32
+// the marching warps take those batches (7.2 / 4.5 us for four of 48^2).
 constexpr int kBatchMarch = 2;
 template <typename T>
 struct BatchShape;
 template <>
 struct BatchShape<float> {
-    static constexpr int TW[kBatchShapes] = {32, 64, 0, 32, 64};
-    static constexpr int TH[kBatchShapes] = {32, 16, 0, 32, 16};
-    static constexpr int NT[kBatchShapes] = {256, 256, 0, 384, 384};
-    static constexpr int MINB[kBatchShapes] = {1, 1, 0, 2, 2};
+    static constexpr int N = 5;
+    static constexpr int TW[N] = {32, 64, 0, 32, 64};
+    static constexpr int TH[N] = {32, 16, 0, 32, 16};
+    static constexpr int NT[N] = {256, 256, 0, 384, 384};
+    static constexpr int MINB[N] = {1, 1, 0, 2, 2};
 };
 template <>
 struct BatchShape<double> {
-    static constexpr int TW[kBatchShapes] = {32, 64, 0, 32, 64};
-    static constexpr int TH[kBatchShapes] = {16, 8, 0, 16, 8};
-    static constexpr int NT[kBatchShapes] = {256, 256, 0, 384, 384};
-    static constexpr int MINB[kBatchShapes] = {1, 1, 0, 2, 2};
+    static constexpr int N = 6;
+    static constexpr int TW[N] = {32, 64, 0, 32, 64, 32};
+    static constexpr int TH[N] = {16, 8, 0, 16, 8, 8};
+    static constexpr int NT[N] = {256, 256, 0, 384, 384, 128};
+    static constexpr int MINB[N] = {1, 1, 0, 2, 2, 1};
 };
 
 struct BatchBase {
@@ -71,6 +76,7 @@ struct BatchEngine final : BatchBase {
     static constexpr int G = kRing;
     using C = cx<T>;
     using SH = BatchShape<T>;
+    static constexpr int kBatchShapes = SH::N;
 
     struct Instance {
         phx_params P{};
@@ -254,7 +260,8 @@ struct BatchEngine final : BatchBase {
         build_march();
         build_one<3>();
         build_one<4>();
-        static_assert(kBatchShapes == 5, "every shape needs its tables");
+        if constexpr (kBatchShapes > 5) build_one<5>();
+        static_assert(kBatchShapes <= 6, "every shape needs its tables");
     }
 
     // ------------------------------------------------------------ launches
@@ -295,7 +302,10 @@ struct BatchEngine final : BatchBase {
             case 1: go<1>(dir); break;
             case kBatchMarch: march.launch(dir, stream); break;
             case 3: go<3>(dir); break;
-            default: go<4>(dir); break;
+            case 4: go<4>(dir); break;
+            default:
+                if constexpr (kBatchShapes > 5) go<5>(dir);
+                break;
         }
         PHX_CUDA(cudaGetLastError());
         ++launches;
