@@ -746,6 +746,10 @@ struct Engine final : EngineBase {
     }
     // ---- TMA-fed persistent variant
     int sm_count = 0;
+    int sms() {
+        if (!sm_count) PHX_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, P.device));
+        return sm_count;
+    }
     std::map<const void*, int> tma_blocks;  // CTAs per SM of each TMA kernel variant
     void tensor_map(CUtensorMap* m, void* alloc_base, bool complex, int box_w_points, int box_h) {
         plane_tensor_map<T>(m, alloc_base, complex, pitch, rows, box_w_points, box_h);
@@ -888,8 +892,22 @@ struct Engine final : EngineBase {
         PHX_CUDA(cudaGetLastError());
         images_ok = true;
     }
+    // the adjoint's sweep: marching warps, or tiles where one round of them holds an
+    // FP64 grid (adj_fused_kernel); PHX_ADJOINT_SWEEP=march / tiles (FP64) forces one
+    static constexpr int kAdjTileW = 32, kAdjTileH = 16;
+    int adj_sweep_forced = [] {
+        const char* e = std::getenv("PHX_ADJOINT_SWEEP");
+        return e && std::string(e) == "march" ? 0 : (e && std::string(e) == "tiles" ? 1 : -1);
+    }();
+    bool adj_tiles() {
+        if (sizeof(T) == 4) return false;
+        if (adj_sweep_forced >= 0) return adj_sweep_forced == 1;
+        const long long tiles =
+            (long long)((N_c + kAdjTileW - 1) / kAdjTileW) * ((N_r + kAdjTileH - 1) / kAdjTileH);
+        return tiles <= sms();
+    }
     // the adjoint's planes need images where its sweep does not wrap
-    bool adj_images() const { return !(adj_fused && AdjMarch<T>::wraps(N_c)); }
+    bool adj_images() { return !(adj_fused && !adj_tiles() && AdjMarch<T>::wraps(N_c)); }
     void go_march(const FusedParams<T>& F, bool res, bool fma, bool store = false) {
         const bool img = march_needs_images(N_c, P.periodic_x) || (store && adj_images());
         if (!store) {
@@ -2443,8 +2461,13 @@ struct Engine final : EngineBase {
                     Q.res = res;
                     cudaEvent_t a = nullptr;
                     prof_begin(a);
-                    if (!sm_count) PHX_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, P.device));
-                    adj_march.launch(Q, sm_count, stream, pdl_on());
+                    if (!adj_tiles()) {
+                        adj_march.launch(Q, sms(), stream, pdl_on());
+                    } else if constexpr (sizeof(T) == 8) {
+                        // launched plainly: no CTA waits in a slot that the second stream could use
+                        dim3 grid((unsigned)((N_c + kAdjTileW - 1) / kAdjTileW), (unsigned)((N_r + kAdjTileH - 1) / kAdjTileH));
+                        adj_fused_kernel<T, kAdjTileW, kAdjTileH, 256><<<grid, 256, 0, stream>>>(Q);
+                    }
                     prof_end(PHX_KERNEL_OTHER, a, (double)N_r * N_c * (5.0 * sizeof(C) + 7.0 * sizeof(T)));
                     ++launches;
                     PHX_CUDA(cudaGetLastError());

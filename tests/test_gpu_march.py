@@ -2,6 +2,7 @@
 (two points per lane), row segments end anywhere.  Against the stage kernels
 (shape 2), bit for bit, and in the fused multiply-add arithmetic against the
 tile kernels (shape 4)."""
+import ctypes
 import itertools
 
 import numpy as np
@@ -9,6 +10,7 @@ import pytest
 
 import bench as B
 import phoenix_b200 as pb
+from phoenix_b200 import _lib as L
 
 pytestmark = pytest.mark.gpu
 
@@ -182,15 +184,18 @@ def test_general_iterations_as_dispatched(require_gpu, monkeypatch, tetm, dtype,
             np.testing.assert_array_equal(x, y, err_msg=f"{n_c} x {n_r}")
 
 
-# the adjoint's vector-Jacobian kernel: strips of 56 columns, wrapping (even
-# widths) and with periodic images (odd ones), against the four-launch form.
+# the adjoint's vector-Jacobian kernels: strips of 56 columns, wrapping (even
+# widths) and with periodic images (odd ones), and the tiles of small FP64 grids,
+# against the four-launch form.
 # FP64: the two differ in the order of a few sums, 1e-12 as in the adjoint's own
 # tests; FP32: 5 iterations of some 100 rounded operations a stage, 2e-5.
+@pytest.mark.parametrize("sweep", ["march", "tiles"])
 @pytest.mark.parametrize("n_c,n_r,dtype,tol", [(8, 8, "f64", 1e-12), (57, 33, "f64", 1e-12), (56, 41, "f64", 1e-12),
                                                (113, 70, "f64", 1e-12), (114, 75, "f32", 2e-5), (58, 9, "f32", 2e-5)])
-def test_adjoint_sweep(require_gpu, monkeypatch, n_c, n_r, dtype, tol):
+def test_adjoint_sweep(require_gpu, monkeypatch, n_c, n_r, dtype, tol, sweep):
     import torch
 
+    monkeypatch.setenv("PHX_ADJOINT_SWEEP", sweep)
     rng = np.random.default_rng([n_c, n_r, 5])
     ct, rt = (torch.complex64, torch.float32) if dtype == "f32" else (torch.complex128, torch.float64)
     z = lambda: torch.tensor(rng.standard_normal((n_r, n_c)) + 1j * rng.standard_normal((n_r, n_c))).to(ct).cuda()  # noqa: E731
@@ -211,3 +216,80 @@ def test_adjoint_sweep(require_gpu, monkeypatch, n_c, n_r, dtype, tol):
             got[stages] = s.adjoint_backward(d_psi, d_n, want_potential=True)
     for a, b in zip(got["0"], got["1"]):
         assert float((a - b).norm() / b.norm()) <= tol
+
+
+# What the backward rests on: stage values stored by the recompute (the marching
+# warps' storing variant in shape 12, tiles in 4, TMA tiles in 10), from checkpoints
+# that the marching iterations left without periodic images, for the sweep that needs
+# none and the one that does; a second run on the same handle, and iterations before
+# the first.  Odd FP64 widths keep their images everywhere.  Tolerances as above, FP32
+# for 7 iterations instead of 5.
+@pytest.mark.parametrize("shape", [12, 4, 10])
+@pytest.mark.parametrize("n_c,n_r,dtype,res,sweep",
+                         [(n_c, n_r, "f64", res, sweep) for sweep in ("march", "tiles")
+                          for n_c, n_r, res in [(56, 41, True), (57, 33, True), (113, 70, False), (9, 8, True)]] +
+                         [(58, 41, "f32", True, "march"), (114, 75, "f32", False, "march")])
+def test_adjoint_recompute(require_gpu, monkeypatch, n_c, n_r, dtype, res, sweep, shape):
+    import torch
+
+    monkeypatch.setenv("PHX_STAGE_SHAPE", str(shape))
+    monkeypatch.setenv("PHX_ADJOINT_SWEEP", sweep)
+    rng = np.random.default_rng([n_c, n_r, 6])
+    ct, rt = (torch.complex64, torch.float32) if dtype == "f32" else (torch.complex128, torch.float64)
+    z = lambda: torch.tensor(rng.standard_normal((n_r, n_c)) + 1j * rng.standard_normal((n_r, n_c))).to(ct).cuda()  # noqa: E731
+    r = lambda: torch.tensor(rng.random((n_r, n_c))).to(rt).cuda()  # noqa: E731
+    psi0, n0, pump, pot, d_psi, d_n = z(), r(), r(), r(), z(), r()
+    got = {}
+    for stages in ("1", "0"):
+        monkeypatch.setenv("PHX_ADJOINT_STAGES", stages)
+        sp = pb.SystemParameters(N_c=n_c, N_r=n_r, L_x=0.3 * n_c, L_y=0.3 * n_r, **B.PHYS, periodic_boundary_x=True,
+                                 periodic_boundary_y=True, dtype=dtype, dt=0.01, t_max=1e12, fft_every=1e12,
+                                 use_reservoir=res, pump_temporal=[pb.Temporal()] if res else [],
+                                 potential_temporal=[pb.Temporal()])
+        with pb.Solver(sp) as s:
+            s.set_field_tensor("potential_plus", pot)
+            s.set_field_tensor("psi_plus", psi0)
+            if res:
+                s.set_field_tensor("pump_plus", pump)
+                s.set_field_tensor("n_plus", n0)
+            s.run(3)
+            got[stages] = []
+            for _ in range(2):
+                s.adjoint_forward(7, 2)
+                got[stages] += [g for g in s.adjoint_backward(d_psi, d_n if res else None, want_pump=res,
+                                                              want_potential=True) if g is not None]
+            got[stages].append(s.get_field_tensor("psi_plus"))
+            assert s.run(1).launch_shape == shape
+    tol = 2.8e-5 if dtype == "f32" else 1e-12
+    assert len(got["0"]) == len(got["1"]) == (9 if res else 5)
+    assert torch.equal(got["0"][-1], got["1"][-1])  # the forward run does not depend on any of this
+    for a, b in zip(got["0"], got["1"]):
+        assert float((a - b).norm() / b.norm()) <= tol
+
+
+# complex envelopes hand an iteration to the stage kernels, which read the periodic
+# images that the marching iterations before it left out; and back again
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+def test_stage_kernels_take_over_from_marching_iterations(require_gpu, monkeypatch, dtype):
+    n_c, n_r, dt = 58, 33, 0.01
+    t = (ctypes.c_double * 6)(0.0, 3.5 * dt, 3.6 * dt, 6.5 * dt, 6.6 * dt, 20 * dt)
+    re = (ctypes.c_double * 6)(1.0, 1.0, 0.8, 0.8, 1.0, 1.0)
+    im = (ctypes.c_double * 6)(0.0, 0.0, 0.5, 0.5, 0.0, 0.0)
+    out = {}
+    for shape in (12, 2):
+        monkeypatch.setenv("PHX_STAGE_SHAPE", str(shape))
+        rng = np.random.default_rng(7)
+        sp = pb.SystemParameters(N_c=n_c, N_r=n_r, L_x=0.3 * n_c, L_y=0.2 * n_r, **B.PHYS, periodic_boundary_x=True,
+                                 periodic_boundary_y=True, dtype=dtype, dt=dt, t_max=1e12, fft_every=1e12,
+                                 pump_temporal=[pb.Temporal()], potential_temporal=[pb.Temporal()])
+        with pb.Solver(sp) as s:
+            L.check(s._lib.phx_set_temporal_table(s._h, L.ENVELOPE["potential"], 0, t, re, im, ctypes.c_int64(6)), s._h)
+            s.set_field("psi_plus", rng.standard_normal((n_r, n_c)) + 1j * rng.standard_normal((n_r, n_c)))
+            s.set_field("n_plus", rng.random((n_r, n_c)))
+            s.set_field("pump_plus", 2.0 * rng.random((n_r, n_c)))
+            s.set_field("potential_plus", 0.3 * rng.standard_normal((n_r, n_c)))
+            launches = [s.run(1).kernel_launches for _ in range(10)]
+            assert shape == 2 or (min(launches) == 1 and max(launches) >= 4 and launches[-1] == 1)
+            out[shape] = [s.get_field("psi_plus"), s.get_field("n_plus")]
+    for a, b in zip(out[12], out[2]):
+        np.testing.assert_array_equal(a, b)
