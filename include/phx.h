@@ -273,7 +273,8 @@ PHX_API phx_status phx_profile_read(phx_handle* h, int32_t kind, double* total_m
  * the request is consumed by the call it stops. */
 PHX_API phx_status phx_request_abort(phx_handle* h);
 
-/* Bound of the one-kernel RK4 iteration's wait for a tile's data (no
+/* Bound of the one-kernel RK4 iteration's wait for a tile's data in its TMA-fed
+ * launch shapes (8-11, 13 and 14; the others wait for nothing) (no
  * reference counterpart): the number of polls of the tile's mbarrier before
  * the wait gives up, also capped at about one second of device clock.  A wait
  * that gives up makes the step return PHX_ERR_TIMEOUT; the iteration's result
@@ -335,8 +336,9 @@ PHX_API phx_status phx_adjoint_backward(phx_handle* h, const void* dpsi_T, const
  * Every instance: scalar RK4, at most one pump and one potential group,
  * constant temporal envelopes, no pulse, no k-space filter, one shared
  * dtype.  One batch iteration advances every instance by one RK4 iteration
- * in a single launch of a persistent kernel that walks the tiles of all
- * instances; phx_batch_step replays a captured CUDA graph of it. */
+ * in a single launch, of a persistent kernel that walks the tiles of all
+ * instances or of marching warps over their row segments, whichever the first
+ * iterations find faster; phx_batch_step replays a captured CUDA graph of it. */
 typedef struct phx_batch phx_batch;
 
 PHX_API phx_status phx_batch_create(const phx_params* instances, int32_t n_instances, phx_batch** out);

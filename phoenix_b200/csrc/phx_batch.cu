@@ -167,6 +167,26 @@ struct BatchEngine final : BatchBase {
     }
 
     // ------------------------------------------------------------ tables
+    // one iteration of an instance from its state plane `dir` into the other
+    FusedParams<T> iteration(Instance& I, int dir) {
+        FusedParams<T> F;
+        std::memset(&F, 0, sizeof(F));
+        fused_constants<T>(F, I.P, I.d, I.dt, I.pitch);
+        // constant temporal envelopes: amplitude 1 at every stage
+        const T cw[4] = {(T)0.0, (T)0.5, (T)0.5, (T)1.0};
+        const std::complex<T> one((T)1, (T)0);
+        for (int s = 0; s < 4; ++s) {
+            F.pump_c[s] = interp<T>(one, one, cw[s]).real();
+            F.pot_c[s] = interp<T>(one, one, cw[s]).real();
+        }
+        F.psi0 = I.cplane(I.psi[dir]);
+        F.psi1 = I.cplane(I.psi[dir ^ 1]);
+        F.n0 = res ? I.rplane(I.n[dir]) : nullptr;
+        F.n1 = res ? I.rplane(I.n[dir ^ 1]) : nullptr;
+        F.pump = I.P.n_pump_groups > 0 ? I.rplane(I.pump) : nullptr;
+        F.pot = I.P.n_potential_groups > 0 ? I.rplane(I.pot) : nullptr;
+        return F;
+    }
     template <int S>
     void table(std::vector<BatchInstance<T>>& hi, std::vector<int>& tiles) {
         constexpr int TW = SH::TW[S], TH = SH::TH[S];
@@ -193,22 +213,7 @@ struct BatchEngine final : BatchBase {
                 plane_tensor_map<T>(&B.maps[dir][1], res ? src_n.p : dummy, false, I.pitch, I.rows, TW + 8, TH + 6);
                 plane_tensor_map<T>(&B.maps[dir][2], B.has_pump ? I.pump.p : dummy, false, I.pitch, I.rows, TW + 8, TH + 6);
                 plane_tensor_map<T>(&B.maps[dir][3], B.has_pot ? I.pot.p : dummy, false, I.pitch, I.rows, TW + 8, TH + 6);
-                FusedParams<T>& F = B.f[dir];
-                std::memset(&F, 0, sizeof(F));
-                fused_constants<T>(F, I.P, I.d, I.dt, I.pitch);
-                // constant temporal envelopes: amplitude 1 at every stage
-                const T cw[4] = {(T)0.0, (T)0.5, (T)0.5, (T)1.0};
-                const std::complex<T> one((T)1, (T)0);
-                for (int s = 0; s < 4; ++s) {
-                    F.pump_c[s] = interp<T>(one, one, cw[s]).real();
-                    F.pot_c[s] = interp<T>(one, one, cw[s]).real();
-                }
-                F.psi0 = I.cplane(I.psi[dir]);
-                F.psi1 = I.cplane(I.psi[dir ^ 1]);
-                F.n0 = res ? I.rplane(I.n[dir]) : nullptr;
-                F.n1 = res ? I.rplane(I.n[dir ^ 1]) : nullptr;
-                F.pump = B.has_pump ? I.rplane(I.pump) : nullptr;
-                F.pot = B.has_pot ? I.rplane(I.pot) : nullptr;
+                B.f[dir] = iteration(I, dir);
             }
         }
     }
@@ -247,11 +252,8 @@ struct BatchEngine final : BatchBase {
         blocks[S] = std::max(1, std::min(n_tiles[S], per_sm * sm_count));
     }
     void build_march() {
-        std::vector<BatchInstance<T>> hi;
-        std::vector<int> tiles;
-        table<0>(hi, tiles);
         std::vector<FusedParams<T>> f;
-        for (const auto& b : hi) f.insert(f.end(), {b.f[0], b.f[1]});
+        for (auto& I : inst) f.insert(f.end(), {iteration(*I, 0), iteration(*I, 1)});
         march.build(f, res, fma, sm_count, stream);
     }
     void build_tables() {

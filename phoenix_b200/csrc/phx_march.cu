@@ -42,8 +42,11 @@ void MarchLauncher<T>::launch(const FusedParams<T>& F, const MarchOptions& o, in
     };
     if (o.store) {
         if (!unit) fail(PHX_ERR_UNSUPPORTED, "stage values are stored with constant envelopes");
-        if (o.res) o.img ? pick_store(true_type{}, true_type{}) : pick_store(true_type{}, false_type{});
-        else o.img ? pick_store(false_type{}, true_type{}) : pick_store(false_type{}, false_type{});
+        auto pick_img = [&](auto img) { o.res ? pick_store(true_type{}, img) : pick_store(false_type{}, img); };
+        if (!o.img) pick_img(false_type{});
+        if constexpr (sizeof(T) == 8) {  // odd numbers of columns, and the tile sweep of the adjoint, are FP64's
+            if (o.img) pick_img(true_type{});
+        }
     } else if (o.fma) {
         if constexpr (sizeof(T) == 4) {
             if (o.res) pick(true_type{}, true_type{}, false_type{});

@@ -20,11 +20,11 @@ template <typename T, int COMPS, int NP, int NV, int NQ, bool NOISE>
 void take(const Variant& v, GeneralKernel<T, COMPS>& k, int& bytes) {
     if (v.np != NP || v.nv != NV || v.nq != NQ || v.noise != NOISE) return;
     constexpr int MINB = COMPS == 1 && sizeof(T) == 4 ? 3 : 2;
-    k = rk4_march_general_kernel<T, COMPS, true, NP, NV, NQ, NOISE, true, false, MINB>;
+    k = rk4_march_general_kernel<T, COMPS, NP, NV, NQ, NOISE, true, false, MINB>;
     if constexpr (sizeof(T) == 8) {  // odd numbers of columns are FP64's
-        if (v.img) k = rk4_march_general_kernel<T, COMPS, true, NP, NV, NQ, NOISE, true, true, MINB>;
+        if (v.img) k = rk4_march_general_kernel<T, COMPS, NP, NV, NQ, NOISE, true, true, MINB>;
     }
-    bytes = MarchGeneralLayout<T, COMPS, true, NP, NV, NQ, NOISE>::bytes;
+    bytes = MarchGeneralLayout<T, COMPS, NP, NV, NQ, NOISE>::bytes;
 }
 template <typename T, int COMPS, int NP, int NV, int NQ>
 void take_noise(const Variant& v, GeneralKernel<T, COMPS>& k, int& bytes) {
@@ -65,7 +65,7 @@ template <typename T>
 const Kind& kind_of(int comps, bool noise) {
     static const Kind f32[4] = {{{2.0, 6.0, {0.456, 0.722, 1.11}}, 0.09, 6.2, 2.4, 2.7, 0.16},
                                 {{2.4, 6.0, {1.15, 1.61, 2.17}}, 0.04, 8.7, 3.2, 4.2, 0.13},
-                                {{2.0, 6.0, {1.08, 1.77, 2.66}}, 0.10, 11.1, 1.4, 6.6, 0.20},
+                                {{2.0, 6.0, {1.08, 1.77, 2.66}}, 0.12, 11.1, 1.4, 6.6, 0.20},
                                 {{3.2, 6.0, {2.73, 3.12, 4.68}}, 0.25, 14.8, 2.5, 8.9, 0.17}};
     static const Kind f64[2] = {{{3.3, 6.0, {0.85, 1.47, 2.21}}, 0.20, 5.7, 1.6, 2.6, 0.19},
                                 {{3.3, 6.0, {1.65, 2.45, 3.68}}, 0.07, 8.6, 1.8, 4.4, 0.11}};

@@ -2537,7 +2537,7 @@ struct Engine final : EngineBase {
         }
         if (want_v) pack_interior_kernel<T><<<256, 256, 0, stream>>>(rplane(vbar), pitch, N_r, N_c, static_cast<T*>(dpot));
         PHX_CUDA(cudaGetLastError());
-        PHX_CUDA(cudaStreamSynchronize(stream));  // scratch planes are freed on return
+        PHX_CUDA(cudaStreamSynchronize(stream));  // both streams' work is done on return
         check_err_flag();
     }
 

@@ -38,7 +38,7 @@ struct MarchGeneralParams {
 // A warp's ring row: per lane 16-byte pieces 512 bytes apart, two points' psi
 // and pulses of every component, the noise values, then the reals (pairs; two
 // pairs to a piece in FP32): n, pump groups, potential groups, noise scale.
-template <typename T, int COMPS, bool RES, int NP, int NV, int NQ, bool NOISE>
+template <typename T, int COMPS, int NP, int NV, int NQ, bool NOISE>
 struct MarchGeneralLayout {
     static constexpr int cx_bytes = 4 * (int)sizeof(T) * 32, per = sizeof(T) == 4 ? 2 : 1;
     static constexpr int psi_off(int q) { return q * cx_bytes; }
@@ -47,9 +47,9 @@ struct MarchGeneralLayout {
     static constexpr int reals_off = xi_off + (NOISE ? cx_bytes : 0);
     static constexpr int real_off(int slot) { return reals_off + slot / per * 512 + slot % per * 8; }
     static constexpr int n_slot(int q) { return q; }
-    static constexpr int pump_slot(int g, int q) { return COMPS * (RES ? 1 : 0) + g * COMPS + q; }
-    static constexpr int pot_slot(int g, int q) { return COMPS * ((RES ? 1 : 0) + NP + g) + q; }
-    static constexpr int scale_slot = COMPS * ((RES ? 1 : 0) + NP + NV);
+    static constexpr int pump_slot(int g, int q) { return COMPS * (1 + g) + q; }
+    static constexpr int pot_slot(int g, int q) { return COMPS * (1 + NP + g) + q; }
+    static constexpr int scale_slot = COMPS * (1 + NP + NV);
     static constexpr int slots = scale_slot + (NOISE ? 1 : 0);
     static constexpr int row_bytes = reals_off + (slots + per - 1) / per * 512;
     static constexpr int warp_bytes = kMarchRing * row_bytes;
@@ -80,10 +80,10 @@ struct MarchSrc {
     __device__ __forceinline__ cx<T> pulse(int g) const { return ps[g][0][j]; }
 };
 
-template <typename T, int COMPS, bool RES, int NP, int NV, int NQ, bool NOISE, bool REALV, bool IMG, int MINB>
+template <typename T, int COMPS, int NP, int NV, int NQ, bool NOISE, bool REALV, bool IMG, int MINB>
 __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
     rk4_march_general_kernel(const __grid_constant__ MarchGeneralParams<T, COMPS> F) {
-    using Lay = MarchGeneralLayout<T, COMPS, RES, NP, NV, NQ, NOISE>;
+    using Lay = MarchGeneralLayout<T, COMPS, NP, NV, NQ, NOISE>;
     using C = cx<T>;
     constexpr int CPT = 2;
     constexpr int PB = 4 * (int)sizeof(T), RB = 2 * (int)sizeof(T);
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
 #pragma unroll
         for (int q = 0; q < COMPS; ++q) {
             copy_cx(d + Lay::psi_off(q), F.psi0[q]);
-            if constexpr (RES) cp_async<RB>(d + Lay::real_off(Lay::n_slot(q)), F.n0[q] + next_g);
+            cp_async<RB>(d + Lay::real_off(Lay::n_slot(q)), F.n0[q] + next_g);
 #pragma unroll
             for (int g = 0; g < NP; ++g)
                 cp_async<RB>(d + Lay::real_off(Lay::pump_slot(g, q)), (q ? F.st[0].pump : P0.pump) + next_g + g * plane);
@@ -142,10 +142,10 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
         auto put_at = [&](int gi) __attribute__((always_inline)) {
             if (store_two) {
                 st_two(out + gi, v);
-                if constexpr (RES) st_two(out_n + gi, nv);
+                st_two(out_n + gi, nv);
             } else {
                 out[gi] = v[0];
-                if constexpr (RES) out_n[gi] = nv[0];
+                out_n[gi] = nv[0];
             }
         };
         if (store_lane && row >= R0) put_at(g);
@@ -160,10 +160,10 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
                 if (store_lane && dx != 0 && c + j < N_c) {
                     const int gi = g + j + dx;
                     out[gi] = v[j];
-                    if constexpr (RES) out_n[gi] = nv[j];
+                    out_n[gi] = nv[j];
                     if (dy) {
                         out[gi + dy * pitch] = v[j];
-                        if constexpr (RES) out_n[gi + dy * pitch] = nv[j];
+                        out_n[gi + dy * pitch] = nv[j];
                     }
                 }
             }
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
 #pragma unroll
         for (int q = 0; q < COMPS; ++q) {
             if constexpr (s > 0) ring_two(ro + Lay::psi_off(q), y0[q]);
-            if constexpr (RES) ring_two(ro + Lay::real_off(Lay::n_slot(q)), n0[q]);
+            ring_two(ro + Lay::real_off(Lay::n_slot(q)), n0[q]);
 #pragma unroll
             for (int g = 0; g < NP; ++g) ring_two(ro + Lay::real_off(Lay::pump_slot(g, q)), pu[g][q]);
 #pragma unroll
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
 #pragma unroll
                 for (int j = 0; j < CPT; ++j) {
                     xi[j] = stage_xi(P, row, c + j);
-                    sc[j] = RES ? scale_of(P, n0[0][j]) : P.noise_scale;
+                    sc[j] = scale_of(P, n0[0][j]);
                     if constexpr (sizeof(T) == 4) {
                         reinterpret_cast<C*>(ro + Lay::xi_off)[j] = xi[j];
                     } else {
@@ -240,10 +240,10 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
 #pragma unroll
             for (int j = 0; j < CPT; ++j) {
                 if constexpr (s == 0) y0[0][j] = ce[0][0][j];
-                const T nin = !RES ? (T)0 : (s == 0 ? n0[0][j] : ns[before][0][j]);
+                const T nin = s == 0 ? n0[0][j] : ns[before][0][j];
                 kn[0][j] = (T)0;
                 const MarchSrc<T, COMPS, NP, NV, NQ, NOISE, REALV> src{pu, po, ps, j};
-                rhs_scalar_src<T, RES>(P, src, ce[s][0][j], up[s][0][j], dn[0][j], j == 0 ? lf[0] : ce[s][0][0],
+                rhs_scalar_src<T, true>(P, src, ce[s][0][j], up[s][0][j], dn[0][j], j == 0 ? lf[0] : ce[s][0][0],
                                        j == 0 ? ce[s][0][1] : rt[0], nin, kw[0][j], kn[0][j]);
             }
         } else {
@@ -277,17 +277,17 @@ __global__ void __launch_bounds__(32 * kMarchWarps, MINB)
                 // the kRk4First / kRk4Mid / kRk4Last sums of the stage kernels
                 if constexpr (s == 0) {
                     t = smul(P.b, kw[q][j]);
-                    if constexpr (RES) tn = rmul(P.b, kn[q][j]);
+                    tn = rmul(P.b, kn[q][j]);
                 } else if constexpr (s < 3) {
                     t = cadd(a[before][q][j], smul(P.b, kw[q][j]));
-                    if constexpr (RES) tn = radd(an[before][q][j], rmul(P.b, kn[q][j]));
+                    tn = radd(an[before][q][j], rmul(P.b, kn[q][j]));
                 }
                 if constexpr (s < 3) {
                     o[q][j] = cadd(y0[q][j], smul(P.dtw, kw[q][j]));
-                    if constexpr (RES) on[q][j] = radd(n0[q][j], rmul(P.dtw, kn[q][j]));
+                    on[q][j] = radd(n0[q][j], rmul(P.dtw, kn[q][j]));
                 } else {
                     o[q][j] = cadd(y0[q][j], smul(P.dt, cadd(a[2][q][j], smul(P.b, kw[q][j]))));
-                    if constexpr (RES) on[q][j] = radd(n0[q][j], rmul(P.dt, radd(an[2][q][j], rmul(P.b, kn[q][j]))));
+                    on[q][j] = radd(n0[q][j], rmul(P.dt, radd(an[2][q][j], rmul(P.b, kn[q][j]))));
                 }
                 if constexpr (NOISE) {
                     // one noise value for both polarisations, scaled by the plus
