@@ -87,9 +87,15 @@ def rk4_alg_bytes_per_point(esz, has_pot=True):
     last = 3 * state + coef + state
     return first + 2 * mid + last
 REF_BIN = os.path.join(ROOT, "oracle", "_ref")
-KERNEL_NAMES = {"rk4_fused": "rk4_fused_kernel / rk4_tma_kernel (whole RK4 iteration)",
-                "rk4_mid": "stage_scalar_kernel<kRk4Mid>", "rk4_first": "stage_scalar_kernel<kRk4First>",
+KERNEL_NAMES = {"rk4_mid": "stage_scalar_kernel<kRk4Mid>", "rk4_first": "stage_scalar_kernel<kRk4First>",
                 "rk4_last": "stage_scalar_kernel<kRk4Last>"}
+
+
+def kernel_name(family, shape):
+    """The kernel behind a family of the library's timing, whole iterations by launch shape."""
+    if family != "rk4_fused":
+        return KERNEL_NAMES.get(family, family)
+    return {12: "rk4_march_kernel", 14: "rk4_stream_kernel"}.get(shape, "rk4_fused_kernel" if shape < 8 else "rk4_tma_kernel")
 
 
 def workload(n, seed=2):
@@ -1000,13 +1006,13 @@ def main():
     alg_launch_bytes = alg_pp * n * n
     achieved = alg_launch_bytes / (per_launch_ms * 1e-3) / 1e9
     traffic = None
-    # DRAM traffic per launch from the committed ncu summary of that kernel at
-    # 4096^2 (the largest case ncu captures here), scaled to this grid by points
+    # DRAM traffic per launch from the committed ncu summary of that kernel on a
+    # larger grid, scaled to this one by points
     tfile = os.path.join(ROOT, "profiles", "traffic_per_point.json")
     if os.path.exists(tfile):
         with open(tfile) as f:
             tj = json.load(f)
-        key = f"{dom_name}_{args.dtype}"
+        key = f"{kernel_name(dom_name, shape)}_{args.dtype}"
         if key in tj:
             traffic = tj[key]["bytes_per_point"] * n * n
     step_bytes = sum(v["bytes"] for k, v in prof.items() if k.startswith("rk4")) / args.steps
@@ -1060,7 +1066,7 @@ def main():
                 "e2e": {"value": e2e_ms * 1e3, "unit": "us/iter", "h2d_bytes_per_step": h2d / e2e_iters,
                         "d2h_bytes_per_step": d2h / e2e_iters},
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                             "frac": achieved / peak, "traffic": traffic, "kernel": KERNEL_NAMES.get(dom_name, dom_name),
+                             "frac": achieved / peak, "traffic": traffic, "kernel": kernel_name(dom_name, shape),
                              "peak_source": peak_src, "alg_bytes_per_point": alg_pp,
                              "alg_bytes_per_launch": alg_launch_bytes,
                              "compulsory_bytes_per_launch": per_launch_bytes,

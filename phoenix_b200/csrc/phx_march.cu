@@ -8,7 +8,7 @@
 namespace phx {
 namespace {
 
-// CTAs per SM the registers must leave room for (FP32 150, FP64 250 registers)
+// CTAs per SM the registers must leave room for (FP32 155, FP64 250 registers)
 template <typename T>
 constexpr int kMarchMinB = sizeof(T) == 4 ? 3 : 2;
 

@@ -15,7 +15,7 @@
 //
 // The strip loses one column a side and stage, so 56 of its columns are stored;
 // a segment of L rows evaluates L + 6, L + 4, L + 2 and L rows.
-// (FP32 150, FP64 250 registers; four points per lane lost to the longer code.)
+// (FP32 155, FP64 250 registers; four points per lane lost to the longer code.)
 //
 // Why: the tile kernels spend their time on stage barriers, on the stencil's
 // shared-memory traffic (70 % of that pipe) and on idle lanes in the
